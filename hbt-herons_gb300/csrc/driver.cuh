@@ -428,7 +428,7 @@ struct IterationDriver
         mem.check(cudaMemsetAsync(O.mbound_type, 0, sizeof(float) * 6 * (size_t)S, st));
       else
       {
-        k_type_masses<<<grid_for((long long)S * kWarp, 256), 256, 0, st>>>(D, O.mbound_type);
+        k_type_masses<<<grid_for(S, 8), 256, 0, st>>>(D, O.mbound_type);
         launches++;
       }
     }

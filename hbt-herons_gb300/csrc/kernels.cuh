@@ -1682,54 +1682,250 @@ __global__ void k_epi_particles(DevState D, KParams K, OutPtrs O, int total)
   segmented_flush<7>(acc7, s, D.com);
 }
 
-// MboundType as CountParticleTypes sums it (src/subhalo.cpp:311-393): per
-// type, float additions in bound order.  One warp per subhalo: the lanes load
-// 32 bound particles at a time (the next 32 while the current ones are
-// added) and lane t replays the additions of type t in order, so the six
-// sums are the reference's sequential ones.
-__global__ void k_type_masses(DevState D, float *out)
+// The binade of a running float sum: `inv` = 1 / spacing of its floats (a
+// power of two), `A` = the sum in units of the spacing.  False where the
+// arithmetic below would leave the normal range (a sum of zero among them).
+__device__ __forceinline__ bool sum_binade(float a, float &inv, unsigned &A)
 {
-  const int s = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (s >= D.S) // whole warps
-    return;
+  const unsigned E = __float_as_uint(a) >> 23; // sign bit included: a negative sum is out of range
+  inv = __uint_as_float((277u - E) << 23);      // 2^23 / 2^(E - 127)
+  A = (__float_as_uint(a) & 0x7fffffu) | 0x800000u;
+  return E >= 30u && E <= 250u;
+}
+
+// A running float sum after a set of masses, without adding them one by one:
+// while the sum stays in one binade (spacing u), fl(a + m) = a + u rint(m / u)
+// unless m / u is halfway between integers, so the additions are one integer
+// sum whatever their order.  units_in_binade gives this lane's rint(m / u)
+// over its masses of one type (row r = 32 consecutive particles, one per
+// lane) and clears `ok` where a mass is negative, huge against u, not finite
+// or a tie.
+constexpr int kTypeRows = 8;
+__device__ __forceinline__ int units_in_binade(int type, const int (&ty)[kTypeRows], const float (&m)[kTypeRows],
+                                               int row0, int rows, float inv, bool &ok)
+{
+  int q = 0;
+#pragma unroll
+  for (int r = 0; r < kTypeRows; r++)
+    if (r >= row0 && r < row0 + rows && ty[r] == type)
+    {
+      const float x = __fmul_rn(m[r], inv), i = rintf(x); // m / u, exact
+      ok = ok && x >= 0.f && x < 65536.f && fabsf(x - i) != 0.5f; // < 2^16 each: 2048 of them fit an int
+      q += ok ? (int)i : 0;
+    }
+  return q;
+}
+
+// sum += Q units; false (sum untouched) when that would leave the binade.
+__device__ __forceinline__ bool add_units(float &sum, unsigned A, int Q)
+{
+  const unsigned T = A + (unsigned)Q;
+  if (T >= 0x1000000u)
+    return false;
+  sum = __uint_as_float((__float_as_uint(sum) & 0xff800000u) | (T & 0x7fffffu));
+  return true;
+}
+
+// One warp adds its rows' masses of one type to the sum, in order.
+__device__ __forceinline__ void add_type_rows(float &sum, int type, const int (&ty)[kTypeRows],
+                                              const float (&m)[kTypeRows])
+{
   const unsigned full = 0xffffffffu;
-  const int st = D.state[s];
-  const int nb = (st == kConverged || st == kMaxIter) ? D.nbound[s] : 0;
-  const long long off = D.off[s];
-  float acc = 0.f;
-  int t = 7;
-  float m = 0.f;
-  if (lane < nb)
+  auto try_rows = [&](int row0, int rows) {
+    float inv;
+    unsigned A;
+    bool ok = sum_binade(sum, inv, A);
+    if (!ok)
+      return false; // the same on every lane
+    const int q = units_in_binade(type, ty, m, row0, rows, inv, ok);
+    return __all_sync(full, ok) && add_units(sum, A, __reduce_add_sync(full, q));
+  };
+  if (try_rows(0, kTypeRows))
+    return;
+#pragma unroll 1
+  for (int r = 0; r < kTypeRows; r++)
   {
-    const int p = D.ord[off + lane];
-    t = D.ty[p] & 7;
-    m = D.pm[p].w;
-  }
-  for (int i0 = 0; i0 < nb; i0 += kWarp)
-  {
-    const int cur_t = t;
-    const float cur_m = m;
-    const int i = i0 + kWarp + lane;
-    t = 7;
-    m = 0.f;
-    if (i < nb)
+    int tr = 7;
+    float mr = 0.f;
+#pragma unroll
+    for (int k = 0; k < kTypeRows; k++)
     {
-      const int p = D.ord[off + i];
-      t = D.ty[p] & 7;
-      m = D.pm[p].w;
+      tr = k == r ? ty[k] : tr;
+      mr = k == r ? m[k] : mr;
     }
-    const int cnt = min(kWarp, nb - i0);
-    for (int q = 0; q < cnt; q++)
+    unsigned left = __ballot_sync(full, tr == type);
+    if (!left || try_rows(r, 1))
+      continue;
+    for (; left; left &= left - 1u)
+      sum = __fadd_rn(sum, __shfl_sync(full, mr, __ffs(left) - 1));
+  }
+}
+
+// MboundType as CountParticleTypes sums it (src/subhalo.cpp:311-393): per
+// type, float additions in bound order, by integer sums within a binade
+// (above).  A block takes eight subhaloes: each warp one of at most
+// kTypeLong bound particles, 256 at a time, then the whole block each longer
+// one, 2048 at a time; only where a type's sum leaves its binade (once per
+// doubling) do the warps add their 256 in turn, and one row of 32 particle by
+// particle.  Bound by the longest subhalo's chain of steps: one warp replaying
+// every addition took 5.3 of the 29.0 ms of a 4e6-particle hydro call (largest
+// subhalo 1.7e5 particles); one warp per subhalo by 256 made that call 26.4
+// ms, blocks by 2048 25.1 ms.  The line at 2048 is where one block step
+// replaces eight warp steps.
+constexpr int kTypeLong = 2048;
+__global__ void __launch_bounds__(256) k_type_masses(DevState D, float *out)
+{
+  __shared__ int s_units[2][8][6];
+  __shared__ int s_bad[2][6]; // bit w: warp w's masses of the type want the slow way
+  __shared__ float s_sum[6];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int s_first = blockIdx.x * 8;
+  auto bound = [&](int s) {
+    const int st = s < D.S ? D.state[s] : (int)kEmpty;
+    return (st == kConverged || st == kMaxIter) ? D.nbound[s] : 0;
+  };
+  auto load = [&](const int *ord, int nb, int i0, int (&t)[kTypeRows], float (&m)[kTypeRows]) {
+    int p[kTypeRows];
+#pragma unroll
+    for (int r = 0; r < kTypeRows; r++)
     {
-      const int tq = __shfl_sync(full, cur_t, q);
-      const float mq = __shfl_sync(full, cur_m, q);
-      if (tq == lane)
-        acc = __fadd_rn(acc, mq);
+      const int i = i0 + r * kWarp + lane;
+      p[r] = i < nb ? ord[i] : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < kTypeRows; r++)
+    {
+      t[r] = p[r] >= 0 ? D.ty[p[r]] & 7 : 7;
+      m[r] = p[r] >= 0 ? D.pm[p[r]].w : 0.f;
+    }
+  };
+  int ty[kTypeRows], nty[kTypeRows];
+  float m[kTypeRows], nm[kTypeRows];
+  auto next = [&]() {
+#pragma unroll
+    for (int r = 0; r < kTypeRows; r++)
+    {
+      ty[r] = nty[r];
+      m[r] = nm[r];
+    }
+  };
+  { // one subhalo per warp
+    const int s = s_first + w, nb = bound(s);
+    if (s < D.S && nb <= kTypeLong)
+    {
+      const int *ord = D.ord + D.off[s];
+      float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}; // the same on every lane
+      load(ord, nb, 0, ty, m);
+      for (int i0 = 0; i0 < nb; i0 += kTypeRows * kWarp)
+      {
+        load(ord, nb, i0 + kTypeRows * kWarp, nty, nm);
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+        {
+          bool has = false;
+#pragma unroll
+          for (int r = 0; r < kTypeRows; r++)
+            has = has || ty[r] == t;
+          if (__any_sync(full, has))
+            add_type_rows(sum[t], t, ty, m);
+        }
+        next();
+      }
+      float v = sum[0];
+#pragma unroll
+      for (int t = 1; t < 6; t++)
+        v = lane == t ? sum[t] : v;
+      if (lane < 6)
+        out[6 * s + lane] = v;
     }
   }
-  if (lane < 6)
-    out[6 * s + lane] = acc;
+  for (int k = 0; k < 8; k++)
+  { // the long ones, by the whole block
+    const int s = s_first + k, nb = bound(s);
+    if (nb <= kTypeLong)
+      continue;
+    const int *ord = D.ord + D.off[s];
+    __syncthreads(); // s_sum of the subhalo before has been written out
+    if (threadIdx.x < 6)
+    {
+      s_sum[threadIdx.x] = 0.f;
+      s_bad[0][threadIdx.x] = 0;
+    }
+    __syncthreads();
+    load(ord, nb, w * kTypeRows * kWarp, ty, m);
+    int par = 0;
+    for (int i0 = 0; i0 < nb; i0 += 256 * kTypeRows, par ^= 1)
+    {
+      load(ord, nb, i0 + 256 * kTypeRows + w * kTypeRows * kWarp, nty, nm);
+#pragma unroll
+      for (int t = 0; t < 6; t++)
+      {
+        float inv;
+        unsigned A;
+        bool ok = sum_binade(s_sum[t], inv, A);
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < kTypeRows; r++)
+          any = any || ty[r] == t;
+        int q = 0;
+        if (__any_sync(full, any))
+        {
+          q = units_in_binade(t, ty, m, 0, kTypeRows, inv, ok);
+          q = __reduce_add_sync(full, q);
+          if (!__all_sync(full, ok) && lane == 0)
+            atomicOr(&s_bad[par][t], 1 << w);
+        }
+        if (lane == 0)
+          s_units[par][w][t] = q;
+      }
+      __syncthreads();
+      unsigned slow = 0u; // types that want the slow way; the same on every thread
+      float sum[6];
+#pragma unroll
+      for (int t = 0; t < 6; t++)
+      {
+        sum[t] = s_sum[t];
+        float inv;
+        unsigned A;
+        sum_binade(sum[t], inv, A);
+        int q = 0;
+#pragma unroll
+        for (int v = 0; v < 8; v++)
+          q += s_units[par][v][t];
+        if (s_bad[par][t] || !add_units(sum[t], A, q))
+          slow |= 1u << t;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0)
+      {
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+          if (!(slow & (1u << t)))
+            s_sum[t] = sum[t];
+      }
+      if (threadIdx.x < 6)
+        s_bad[par ^ 1][threadIdx.x] = 0;
+      for (int v = 0; slow && v < 8; v++)
+      { // the warps in turn
+        __syncthreads();
+        if (w == v)
+#pragma unroll
+          for (int t = 0; t < 6; t++)
+            if (slow & (1u << t))
+            {
+              float a = s_sum[t];
+              add_type_rows(a, t, ty, m);
+              if (lane == 0)
+                s_sum[t] = a;
+            }
+      }
+      __syncthreads();
+      next();
+    }
+    if (threadIdx.x < 6)
+      out[6 * s + threadIdx.x] = s_sum[threadIdx.x];
+  }
 }
 
 // Scalar outputs of each subhalo (one thread per subhalo): kinematics, type
