@@ -144,6 +144,7 @@ enum Slot
   S_PR_OFF, S_PR_CNT, S_PR_FIN, S_PR_RR, S_PR_MM, S_PR_K, S_PR_V, S_PR_KA, S_PR_VA, S_PR_MC, S_PR_VK, S_PR_SO,
   S_PR_SH, S_PR_SCR, S_PR_POS, S_PR_MASS, S_PR_ORD, S_PR_NB, S_PR_MBND, S_PR_MBP, S_PR_OUTF, S_PR_OUTI, S_PR_OUTL,
   S_RE_OFF, S_RE_SG, S_RE_GP, S_RE_FL, S_RE_RK, S_RE_TG, S_RE_TS, S_RE_GO, S_RE_POS, S_RE_TY, S_RE_DEST,
+  S_RE_QK, S_RE_QKA, S_RE_QV, S_RE_QVA,
   S_NUM
 };
 
@@ -1297,9 +1298,31 @@ int reassign_run(hbtg_handle *H, const hbtg_params *p, const hbtg_reassign *r, i
   const int src_total = R.scan_counts(D.src_cnt, D.src_off, G);
   if (src_total > 0)
     R.build_tree(src_total, true);
-  if (N > 0)
+  HBTG_CUDA(cudaMemsetAsync(Q.dest, 0xff, sizeof(long long) * (size_t)N, st)); // -1: stays
+  const long long nq = N - T;
+  if (nq > 0 && src_total > 0)
   {
-    k_re_query<<<blocks_for(N, 128), 128, 0, st>>>(Q, D, N);
+    uint32_t *qval = P.get<uint32_t>(S_RE_QV, (size_t)nq), *qval_alt = P.get<uint32_t>(S_RE_QVA, (size_t)nq);
+    unsigned long long *qkey = P.get<unsigned long long>(S_RE_QK, (size_t)nq),
+                       *qkey_alt = P.get<unsigned long long>(S_RE_QKA, (size_t)nq);
+    Q.qkey = qkey;
+    Q.qval = qval;
+    k_re_queries<<<blocks_for(N, 256), 256, 0, st>>>(Q, D, N);
+    launches++;
+    if (radix_sort_pairs<unsigned long long>(qkey, qval, qkey_alt, qval_alt, nq, 0, 3 * kReDigits + bits,
+                                             mem.radix_table(nq), mem.radix_scan_scratch(nq), st, &launches))
+    {
+      Q.qkey = qkey_alt;
+      Q.qval = qval_alt;
+    }
+    const unsigned qb = blocks_for(nq, 128);
+    const ReRadii radii(Q.r0);
+    if (k <= 8) // the lists sized for the neighbours asked for
+      k_re_query<8><<<qb, 128, 0, st>>>(Q, D, radii, nq);
+    else if (k <= 16)
+      k_re_query<16><<<qb, 128, 0, st>>>(Q, D, radii, nq);
+    else
+      k_re_query<kMaxNeighbours><<<qb, 128, 0, st>>>(Q, D, radii, nq);
     launches++;
   }
   R.check();
