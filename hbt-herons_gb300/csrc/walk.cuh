@@ -26,12 +26,20 @@
 //               the rest, and "near" ones.  Whenever a list fills, every lane reads each
 //               entry (a shared-memory broadcast) and adds the term of the
 //               entries its mask bit selects: -m / r for the far list with no
-//               branch, two entries at a time in packed FP32x2 arithmetic
-//               (each half an IEEE FP32 operation, so the same values as
-//               scalar code), and the cubic-spline softened kernel where
-//               r < h for the near list.  Lists are padded to a multiple of
+//               branch, and the cubic-spline softened kernel where r < h for
+//               the near list.  Distances are formed two entries at a time in
+//               packed FP32x2 arithmetic (each half an IEEE FP32 operation, so
+//               the same values as scalar code).  Lists are padded to a multiple of
 //               eight with massless entries; blocks of eight terms are summed
 //               in FP32 and Kahan-added to the potential.
+//
+// Periodic wrap.  A wrapped separation is a - b, (a - box) - b or a -
+// (b - box) (sep), and along each axis the box of 32 neighbouring targets
+// nearly always takes one of the three for all of them.  Then the entry is
+// stored as a or a - box, with a flag where the targets are to be taken as
+// b - box, and it costs what an unwrapped one does; a cell's opening test by
+// the box and the packed tests work on the same coordinates.  Only an entry
+// that some targets wrap and others do not goes target by target.
 //
 // Opening test.  The reference opens a cell when len^2 > r^2 theta^2, with
 // len^2 in float and r^2 in double from the float coordinates
@@ -56,6 +64,16 @@
 // index strictly or shrinks the pending list.
 // A node's second slot is read for leaves too: the tree array carries one
 // padding slot after its last slot.
+//
+// Bound by instruction issue (79 % of the slots at 28 warps per SM), a little
+// over half of it in the traversal.  So a step has one path for every lane
+// (lanes without a range read the last one again), the three lists share one
+// layout and one write, a warp's arrays lie together behind one base address,
+// and the far terms use the reciprocal square root without the steps for
+// subnormal arguments.  Against a version with separate lists, per-kind
+// branches and rsqrtf, on the 5e7-particle learned batch: 137.4 -> 123.7 ms a
+// call; on a 5e6-particle plain batch with a halo across a box face 31.1 ->
+// 29.0 ms (walk 20.9 -> 16.6 ms); a subsampled hydro call 23.5 -> 21.0 ms.
 #pragma once
 
 #include "kernels.cuh"
@@ -105,26 +123,24 @@ __device__ __forceinline__ void tick(WalkCount &cnt, int q, long long &t, int la
   t = now;
 }
 
-struct WalkShared
+// Entry lists of one warp, in one array of pairs (a = (x0, x1, y0, y1),
+// b = (z0, z1, -m0, -m1), two entries per packed operation): the far entries
+// that every target takes, the other far entries, the near ones.  The last
+// two have target masks; a wrapped walk, which lists every entry as near,
+// keeps its wrap flags in the far list's words.
+constexpr int kFarAt = kWalkFull, kNearAt = kWalkFull + kWalkFar, kWalkEntries = kNearAt + kWalkNear;
+
+// Everything of a warp lies together, so one base address serves it all.
+struct WalkWarp
 {
-  // far list, two entries per pair (packed FP32x2 evaluation): fa = (x0, x1,
-  // y0, y1), fb = (z0, z1, m0, m1), fm = the two entries' target masks
-  float4 fa[kWalkWarps][kWalkFar / 2];
-  float4 fb[kWalkWarps][kWalkFar / 2];
-  uint2 fm[kWalkWarps][kWalkFar / 2];
-  // far list of entries that every target takes: ga = (x0, x1, y0, y1),
-  // gb = (z0, z1, -m0, -m1)
-  float4 ga[kWalkWarps][kWalkFull / 2];
-  float4 gb[kWalkWarps][kWalkFull / 2];
-  float4 near[kWalkWarps][kWalkNear];
-  unsigned nmsk[kWalkWarps][kWalkNear];
-  int ia[kWalkWarps][kWalkStack];       // range: first slot
-  int ie[kWalkWarps][kWalkStack];       //        end slot
-  unsigned im[kWalkWarps][kWalkStack];  //        targets still walking it
-  int pa[kWalkWarps][kWalkPending];     // pending cell: slot
-  unsigned pm[kWalkWarps][kWalkPending]; //              targets that reach it
-  float4 txy[kWalkWarps][kWalkWarp2];   // targets, negated, in pairs: (x0, x1, y0, y1)
-  float2 tz[kWalkWarps][kWalkWarp2];    //                             (z0, z1)
+  float4 a[kWalkEntries / 2];
+  float4 b[kWalkEntries / 2];
+  unsigned mask[kWalkFar + kWalkNear];
+  int2 ie[kWalkStack];      // range: first slot, end slot
+  unsigned im[kWalkStack];  //        targets still walking it
+  int2 pend[kWalkPending];  // pending cell: slot, targets that reach it
+  float4 txy[kWalkWarp2];   // targets, negated, in pairs: (x0, x1, y0, y1)
+  float2 tz[kWalkWarp2];    //                             (z0, z1)
 };
 
 // a - b, with the periodic wrap of NEAREST (src/config_parser.h:218-219)
@@ -147,16 +163,15 @@ __device__ __forceinline__ float dist2(float dx, float dy, float dz)
 
 // The reference's opening decision in its own arithmetic: float len^2
 // against r^2 theta^2 in double, r^2 from the float coordinates.
-template <bool Wrap>
 __device__ __noinline__ bool opens_exact(float cx, float cy, float cz, float lenf, float tx, float ty, float tz,
-                                         const KParams &K)
+                                         int periodic, float box, float half, float theta2)
 {
   double d[3] = {(double)cx - (double)tx, (double)cy - (double)ty, (double)cz - (double)tz}; // exact
-  if (K.periodic)
+  if (periodic)
     for (int q = 0; q < 3; q++)
-      d[q] = nearest_d(d[q], (double)K.half, (double)K.box);
+      d[q] = nearest_d(d[q], (double)half, (double)box);
   const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
-  return (double)__fmul_rn(lenf, lenf) > __dmul_rn(r2, (double)K.theta2);
+  return (double)__fmul_rn(lenf, lenf) > __dmul_rn(r2, (double)theta2);
 }
 
 // One target's test of a cell (centre c, threshold crit = len^2/theta^2).
@@ -169,7 +184,7 @@ __device__ __forceinline__ bool target_opens(float cx, float cy, float cz, float
     return true;
   if (r2 > __fmul_rn(crit, kBandHi))
     return false;
-  return opens_exact<Wrap>(cx, cy, cz, lenf, tx, ty, tz, K);
+  return opens_exact(cx, cy, cz, lenf, tx, ty, tz, K.periodic, K.box, K.half, K.theta2);
 }
 
 // Target t of the warp from the negated pairs.
@@ -184,42 +199,56 @@ __device__ __forceinline__ void target_at(const float4 *txy, const float2 *tz, i
 }
 
 // Every target's own decision on one cell (centre c, threshold crit, side
-// lenf): bit t set when target t (of the mask m) opens it.  Without the wrap,
-// two targets per packed operation; each half is the FP32 operation of
-// target_opens (c + (-t) is c - t exactly), so the decisions are the same.
+// lenf): bit t set when target t (of the mask m) opens it.  Two targets per
+// packed operation; each half is the FP32 operation of target_opens (c + (-t)
+// is c - t exactly), so the decisions are the same; the sign of r^2 minus the
+// band's edge is the comparison, shifted into the mask (r^2 = NaN, from
+// coordinates that are not finite, decides nothing of use either way).  With
+// Wrap, c is the cell as all targets see it (wrap_cell) and a target's
+// coordinate along the axes of `flags` is taken less one box.
 template <bool Wrap>
 __device__ __forceinline__ unsigned opens_mask(const float4 *txy, const float2 *tz, float cx, float cy, float cz,
-                                               float crit, float lenf, unsigned m, const KParams &K)
+                                               float crit, float lenf, unsigned m, unsigned flags, float ox, float oy,
+                                               float oz, const KParams &K)
 {
-  unsigned O = 0u;
-  if (Wrap)
-  {
-    for (unsigned r = m; r; r &= r - 1u)
-    {
-      const int t = __ffs(r) - 1;
-      float tx, ty, tzz;
-      target_at(txy, tz, t, tx, ty, tzz);
-      if (target_opens<true>(cx, cy, cz, crit, lenf, tx, ty, tzz, K))
-        O |= 1u << t;
-    }
-    return O;
-  }
   const float lo = __fmul_rn(crit, kBandLo), hi = __fmul_rn(crit, kBandHi);
   const float2 c_x = make_float2(cx, cx), c_y = make_float2(cy, cy), c_z = make_float2(cz, cz);
-  unsigned B = 0u; // not beyond the band's far edge
+  const float2 nlo = make_float2(-lo, -lo), nhi = make_float2(-hi, -hi);
+  unsigned O = 0u, B = 0u; // nearer than the band; not beyond the band's far edge
 #pragma unroll
-  for (int q = 0; q < kWalkWarp2; q++)
+  for (int q = kWalkWarp2 - 1; q >= 0; q--)
   {
-    const float4 P = txy[q];
-    const float2 Z = tz[q];
+    float4 P = txy[q];
+    float2 Z = tz[q];
+    if (Wrap && flags)
+    { // -(t - box), rounded as t - box is
+      if (flags & 1u)
+      {
+        P.x = __fadd_rn(P.x, K.box);
+        P.y = __fadd_rn(P.y, K.box);
+      }
+      if (flags & 2u)
+      {
+        P.z = __fadd_rn(P.z, K.box);
+        P.w = __fadd_rn(P.w, K.box);
+      }
+      if (flags & 4u)
+      {
+        Z.x = __fadd_rn(Z.x, K.box);
+        Z.y = __fadd_rn(Z.y, K.box);
+      }
+    }
     const float2 dx = __fadd2_rn(c_x, make_float2(P.x, P.y));
     const float2 dy = __fadd2_rn(c_y, make_float2(P.z, P.w));
     const float2 dz = __fadd2_rn(c_z, Z);
     float2 r2 = __fmul2_rn(dx, dx);
     r2 = __ffma2_rn(dy, dy, r2);
     r2 = __ffma2_rn(dz, dz, r2);
-    O |= (r2.x < lo ? 1u : 0u) << (2 * q) | (r2.y < lo ? 2u : 0u) << (2 * q);
-    B |= (r2.x > hi ? 0u : 1u) << (2 * q) | (r2.y > hi ? 0u : 2u) << (2 * q);
+    const float2 u = __fadd2_rn(r2, nlo), v = __fadd2_rn(nhi, r2);
+    O = __funnelshift_l(__float_as_uint(u.y), O, 1); // (O << 1) | (r2.y < lo)
+    O = __funnelshift_l(__float_as_uint(u.x), O, 1);
+    B = __funnelshift_l(__float_as_uint(v.y), B, 1); // (B << 1) | (r2.y < hi)
+    B = __funnelshift_l(__float_as_uint(v.x), B, 1);
   }
   O &= m;
   // inside the band: the reference's double arithmetic
@@ -228,19 +257,64 @@ __device__ __forceinline__ unsigned opens_mask(const float4 *txy, const float2 *
     const int t = __ffs(r) - 1;
     float tx, ty, tzz;
     target_at(txy, tz, t, tx, ty, tzz);
-    if (opens_exact<false>(cx, cy, cz, lenf, tx, ty, tzz, K))
+    if (opens_exact(ox, oy, oz, lenf, tx, ty, tzz, K.periodic, K.box, K.half, K.theta2))
       O |= 1u << t;
   }
   return O;
 }
 
-// Squared distance from a point to the targets' bounding box.
-__device__ __forceinline__ float box_gap2(const float *lo, const float *hi, float x, float y, float z)
+// The same one target at a time, for a cell that some targets wrap and others
+// do not.
+__device__ __forceinline__ unsigned opens_mask_each(const float4 *txy, const float2 *tz, float cx, float cy, float cz,
+                                                    float crit, float lenf, unsigned m, const KParams &K)
 {
-  const float g[3] = {fmaxf(fmaxf(__fsub_rn(lo[0], x), __fsub_rn(x, hi[0])), 0.f),
-                      fmaxf(fmaxf(__fsub_rn(lo[1], y), __fsub_rn(y, hi[1])), 0.f),
-                      fmaxf(fmaxf(__fsub_rn(lo[2], z), __fsub_rn(z, hi[2])), 0.f)};
-  return dist2(g[0], g[1], g[2]);
+  unsigned O = 0u;
+  for (unsigned r = m; r; r &= r - 1u)
+  {
+    const int t = __ffs(r) - 1;
+    float tx, ty, tzz;
+    target_at(txy, tz, t, tx, ty, tzz);
+    if (target_opens<true>(cx, cy, cz, crit, lenf, tx, ty, tzz, K))
+      O |= 1u << t;
+  }
+  return O;
+}
+
+// Axis by axis, how the targets' box [lo, hi] wraps against coordinate c
+// (sep's comparisons at the box's ends; c - t is monotonic in t): returns the
+// coordinate to store and adds to `flags` bit d where the targets are taken
+// less one box, or kMixed where they differ.
+constexpr unsigned kMixed = 8u;
+__device__ __forceinline__ float wrap_axis(float c, float lo, float hi, int d, unsigned &flags, const KParams &K)
+{
+  const float dmin = __fsub_rn(c, hi), dmax = __fsub_rn(c, lo);
+  if (dmin > K.half)
+    return __fsub_rn(c, K.box);
+  if (dmax < -K.half)
+    flags |= 1u << d;
+  else if (dmax > K.half || dmin < -K.half)
+    flags |= kMixed;
+  return c;
+}
+
+// Smallest and largest squared distance from a point to the targets' box.
+__device__ __forceinline__ void box_dist2(const float *lo, const float *hi, float x, float y, float z, float &near2,
+                                          float &far2)
+{
+  const float l[3] = {__fsub_rn(lo[0], x), __fsub_rn(lo[1], y), __fsub_rn(lo[2], z)};
+  const float h[3] = {__fsub_rn(x, hi[0]), __fsub_rn(y, hi[1]), __fsub_rn(z, hi[2])};
+  near2 = dist2(fmaxf(fmaxf(l[0], h[0]), 0.f), fmaxf(fmaxf(l[1], h[1]), 0.f), fmaxf(fmaxf(l[2], h[2]), 0.f));
+  far2 = dist2(fmaxf(fabsf(l[0]), fabsf(h[0])), fmaxf(fabsf(l[1]), fabsf(h[1])), fmaxf(fabsf(l[2]), fabsf(h[2])));
+}
+
+// 1 / sqrt of a number that is not subnormal: the approximation that rsqrtf
+// returns there, without the steps that scale a subnormal argument (three of
+// its four instructions).
+__device__ __forceinline__ float rsqrt_normal(float x)
+{
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
 // The potential term of one entry for one target at squared distance r2.
@@ -261,48 +335,53 @@ __device__ __forceinline__ void kahan_add(float &sum, float &comp, float v)
 // loops need no guard).
 constexpr float kFarAway = 3e18f;
 
-// Pads a list to a multiple of eight with massless entries; returns the
-// padded length.  The caller leaves room for seven more entries.
-__device__ __forceinline__ int pad8(float4 *ent, unsigned *msk, int n, int lane)
+// Writes entry k (pair layout).
+__device__ __forceinline__ void entry_put(float4 *ea, float4 *eb, int k, float x, float y, float z, float nm)
+{
+  float *A = reinterpret_cast<float *>(ea + (k >> 1)) + (k & 1), *B = reinterpret_cast<float *>(eb + (k >> 1)) + (k & 1);
+  A[0] = x;
+  A[2] = y;
+  B[0] = z;
+  B[2] = nm;
+}
+
+// Pads the list that starts at entry `at` and holds n to a multiple of eight
+// with massless entries; returns the padded length.  The caller leaves room
+// for seven more entries.
+__device__ __forceinline__ int pad8(float4 *ea, float4 *eb, unsigned *mask, int at, int n, int lane)
 {
   const int padded = (n + 7) & ~7;
   if (n + lane < padded)
   {
-    ent[n + lane] = make_float4(kFarAway, kFarAway, kFarAway, 0.f);
-    msk[n + lane] = 0u;
+    entry_put(ea, eb, at + n + lane, kFarAway, kFarAway, kFarAway, 0.f);
+    if (at >= kFarAt)
+      mask[at - kFarAt + n + lane] = 0u;
   }
   __syncwarp();
   return padded;
 }
 
-// Writes far-list entry k (pair layout).
-__device__ __forceinline__ void far_put(float4 *fa, float4 *fb, uint2 *fm, int k, float x, float y, float z, float m,
-                                        unsigned mask)
+// Squared distances of entry pair (A, B) from a target (negated coordinates,
+// entry + (-target) is exact as a subtraction).
+__device__ __forceinline__ float2 pair_r2(const float4 &A, const float4 &B, float2 ntx, float2 nty, float2 ntz)
 {
-  float *A = reinterpret_cast<float *>(fa + (k >> 1)), *B = reinterpret_cast<float *>(fb + (k >> 1));
-  const int h = k & 1;
-  A[h] = x;
-  A[2 + h] = y;
-  B[h] = z;
-  B[2 + h] = m;
-  reinterpret_cast<unsigned *>(fm + (k >> 1))[h] = mask;
+  const float2 dx = __fadd2_rn(make_float2(A.x, A.y), ntx);
+  const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nty);
+  const float2 dz = __fadd2_rn(make_float2(B.x, B.y), ntz);
+  float2 r2 = __fmul2_rn(dx, dx);
+  r2 = __ffma2_rn(dy, dy, r2);
+  return __ffma2_rn(dz, dz, r2);
 }
 
-__device__ __forceinline__ int pad8_far(float4 *fa, float4 *fb, uint2 *fm, int n, int lane)
-{
-  const int padded = (n + 7) & ~7;
-  if (n + lane < padded)
-    far_put(fa, fb, fm, n + lane, kFarAway, kFarAway, kFarAway, 0.f, 0u);
-  __syncwarp();
-  return padded;
-}
-
-// Far list: every target is at least one softening length from every entry
-// (never used for wrapped subhaloes).  Two entries per packed operation.
-__device__ __forceinline__ void eval_far(const float4 *fa, const float4 *fb, const uint2 *fm, int n, unsigned lanebit,
-                                         float tx, float ty, float tz, float &sum, float &comp)
+// Far lists: every target is at least one softening length from every entry
+// (never used for wrapped subhaloes).  Masked: only the targets of an entry's
+// mask take it.
+template <bool Masked>
+__device__ __forceinline__ void eval_far(const float4 *ea, const float4 *eb, const unsigned *mask, int n,
+                                         unsigned lanebit, float tx, float ty, float tz, float &sum, float &comp)
 {
   const float2 ntx = make_float2(-tx, -tx), nty = make_float2(-ty, -ty), ntz = make_float2(-tz, -tz);
+  const uint2 *fm = reinterpret_cast<const uint2 *>(mask);
   for (int i = 0; i < n; i += 8)
   {
     float2 acc = make_float2(0.f, 0.f);
@@ -310,91 +389,77 @@ __device__ __forceinline__ void eval_far(const float4 *fa, const float4 *fb, con
     for (int q = 0; q < 4; q++)
     {
       const int pp = (i >> 1) + q;
-      const float4 A = fa[pp], B = fb[pp];
-      const uint2 mk = fm[pp];
-      const float2 dx = __fadd2_rn(make_float2(A.x, A.y), ntx); // entry - target, exact as a subtraction
-      const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nty);
-      const float2 dz = __fadd2_rn(make_float2(B.x, B.y), ntz);
-      float2 r2 = __fmul2_rn(dx, dx);
-      r2 = __ffma2_rn(dy, dy, r2);
-      r2 = __ffma2_rn(dz, dz, r2);
-      const float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-      const float2 nm = make_float2((mk.x & lanebit) ? -B.z : 0.f, (mk.y & lanebit) ? -B.w : 0.f);
+      const float4 A = ea[pp], B = eb[pp];
+      const float2 r2 = pair_r2(A, B, ntx, nty, ntz);
+      const float2 rs = make_float2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
+      float2 nm = make_float2(B.z, B.w);
+      if (Masked)
+      {
+        const uint2 mk = fm[pp];
+        nm = make_float2((mk.x & lanebit) ? B.z : 0.f, (mk.y & lanebit) ? B.w : 0.f);
+      }
       acc = __ffma2_rn(nm, rs, acc);
     }
     kahan_add(sum, comp, acc.x + acc.y);
   }
 }
 
-// Writes entry k of the far list that every target takes.
-__device__ __forceinline__ void full_put(float4 *ga, float4 *gb, int k, float x, float y, float z, float m)
+// One near entry's term: the softened form only when some lane is inside the
+// softening length (its square root and polynomial are skipped otherwise).
+// h2s >= h2 keeps subnormal r2 out of rsqrt_normal.
+__device__ __forceinline__ float near_term(float nm, float r2, const KParams &K, float h2, float h2s)
 {
-  float *A = reinterpret_cast<float *>(ga + (k >> 1)), *B = reinterpret_cast<float *>(gb + (k >> 1));
-  const int h = k & 1;
-  A[h] = x;
-  A[2 + h] = y;
-  B[h] = z;
-  B[2 + h] = -m;
-}
-
-__device__ __forceinline__ int pad8_full(float4 *ga, float4 *gb, int n, int lane)
-{
-  const int padded = (n + 7) & ~7;
-  if (n + lane < padded)
-    full_put(ga, gb, n + lane, kFarAway, kFarAway, kFarAway, 0.f);
-  __syncwarp();
-  return padded;
-}
-
-// The far list that every target takes: no per-entry selection.
-__device__ __forceinline__ void eval_full(const float4 *ga, const float4 *gb, int n, float tx, float ty, float tz,
-                                          float &sum, float &comp)
-{
-  const float2 ntx = make_float2(-tx, -tx), nty = make_float2(-ty, -ty), ntz = make_float2(-tz, -tz);
-  for (int i = 0; i < n; i += 8)
-  {
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-    {
-      const int pp = (i >> 1) + q;
-      const float4 A = ga[pp], B = gb[pp];
-      const float2 dx = __fadd2_rn(make_float2(A.x, A.y), ntx);
-      const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nty);
-      const float2 dz = __fadd2_rn(make_float2(B.x, B.y), ntz);
-      float2 r2 = __fmul2_rn(dx, dx);
-      r2 = __ffma2_rn(dy, dy, r2);
-      r2 = __ffma2_rn(dz, dz, r2);
-      const float2 rs = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-      acc = __ffma2_rn(make_float2(B.z, B.w), rs, acc);
-    }
-    kahan_add(sum, comp, acc.x + acc.y);
-  }
+  if (__any_sync(0xffffffffu, r2 < h2s))
+    return softened_term(-nm, r2, K, h2);
+  return nm * rsqrt_normal(r2);
 }
 
 // Near list: the softened kernel where r < h (src/gravity_tree.cpp:150-162).
+// With Wrap, `flags` holds how the targets take each entry (wrap_axis).
 template <bool Wrap>
-__device__ __forceinline__ void eval_near(const float4 *ent, const unsigned *msk, int n, unsigned lanebit, float tx,
-                                          float ty, float tz, const KParams &K, float h2, float &sum, float &comp)
+__device__ __forceinline__ void eval_near(const float4 *ea, const float4 *eb, const unsigned *mask,
+                                          const unsigned *flags, int n, unsigned lanebit, float tx, float ty, float tz,
+                                          const KParams &K, float h2, float h2s, float &sum, float &comp)
 {
-  const unsigned full = 0xffffffffu;
+  const float2 ntx = make_float2(-tx, -tx), nty = make_float2(-ty, -ty), ntz = make_float2(-tz, -tz);
+  const uint2 *nm2 = reinterpret_cast<const uint2 *>(mask), *nf2 = reinterpret_cast<const uint2 *>(flags);
   for (int i = 0; i < n; i += 8)
   {
     float part = 0.f;
-#pragma unroll 2
-    for (int u = 0; u < 8; u++)
+#pragma unroll 1
+    for (int q = 0; q < 4; q++)
     {
-      const float4 e = ent[i + u];
-      const float m = (msk[i + u] & lanebit) ? e.w : 0.f;
-      const float r2 = dist2(sep<Wrap>(e.x, tx, K), sep<Wrap>(e.y, ty, K), sep<Wrap>(e.z, tz, K));
-      // the softened form only when some lane is inside the softening length
-      // (its square root and polynomial are skipped otherwise)
-      float t;
-      if (__any_sync(full, r2 < h2))
-        t = softened_term(m, r2, K, h2);
+      const int pp = (i >> 1) + q;
+      const float4 A = ea[pp], B = eb[pp];
+      const uint2 mk = nm2[pp];
+      float2 r2;
+      if (Wrap)
+      {
+        const uint2 f = nf2[pp];
+        if ((f.x | f.y) == 0u)
+          r2 = pair_r2(A, B, ntx, nty, ntz);
+        else
+        {
+          float r[2];
+#pragma unroll
+          for (int e = 0; e < 2; e++)
+          {
+            const unsigned fe = e ? f.y : f.x;
+            const float ex = e ? A.y : A.x, ey = e ? A.w : A.z, ez = e ? B.y : B.x;
+            if (fe & kMixed)
+              r[e] = dist2(sep<true>(ex, tx, K), sep<true>(ey, ty, K), sep<true>(ez, tz, K));
+            else
+              r[e] = dist2(__fsub_rn(ex, (fe & 1u) ? __fsub_rn(tx, K.box) : tx),
+                           __fsub_rn(ey, (fe & 2u) ? __fsub_rn(ty, K.box) : ty),
+                           __fsub_rn(ez, (fe & 4u) ? __fsub_rn(tz, K.box) : tz));
+          }
+          r2 = make_float2(r[0], r[1]);
+        }
+      }
       else
-        t = -m * rsqrtf(r2);
-      part += t;
+        r2 = pair_r2(A, B, ntx, nty, ntz);
+      part += near_term((mk.x & lanebit) ? B.z : 0.f, r2.x, K, h2, h2s);
+      part += near_term((mk.y & lanebit) ? B.w : 0.f, r2.y, K, h2, h2s);
     }
     kahan_add(sum, comp, part);
   }
@@ -439,16 +504,15 @@ __device__ __forceinline__ void walk_range(const float4 *__restrict__ T, int a, 
 // Potentials of the (up to) 32 targets of chunk c.
 template <bool Wrap, bool Count>
 __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, int s, int root, int lane, bool valid,
-                                           int p, float4 x, float self, WalkShared &sh, int w, WalkCount &cnt)
+                                           int p, float4 x, float self, WalkWarp &sh, WalkCount &cnt)
 {
   const float4 *__restrict__ T = D.nodes;
-  float4 *fa = sh.fa[w], *fb = sh.fb[w], *nea = sh.near[w], *ga = sh.ga[w], *gb = sh.gb[w];
-  uint2 *fm = sh.fm[w];
-  unsigned *nmsk = sh.nmsk[w];
-  int *ia = sh.ia[w], *ie = sh.ie[w];
-  unsigned *im = sh.im[w];
+  float4 *ea = sh.a, *eb = sh.b;
+  unsigned *mask = sh.mask;
+  int2 *ie = sh.ie, *pend = sh.pend;
+  unsigned *im = sh.im;
   const unsigned full = 0xffffffffu, lanebit = 1u << lane, below = lanebit - 1u;
-  const float h2 = K.h * K.h;
+  const float h2 = K.h * K.h, h2s = fmaxf(h2, 1.17549435e-38f); // far entries: r^2 not subnormal
   long long t_all = Count ? clock64() : 0, t = t_all;
   const unsigned vmask = __ballot_sync(full, valid);
   // bounding box of the targets
@@ -465,20 +529,17 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
   float sum = valid ? self / K.soft : 0.f, comp = 0.f;
   if (lane == 0)
   {
-    ia[0] = root;
-    ie[0] = __float_as_int(__ldg(&T[root + 1]).y);
+    ie[0] = make_int2(root, __float_as_int(__ldg(&T[root + 1]).y));
     im[0] = vmask;
   }
   // the targets, negated, in pairs (the pending cells' tests read them)
   {
-    float *X = reinterpret_cast<float *>(sh.txy[w]), *Z = reinterpret_cast<float *>(sh.tz[w]);
+    float *X = reinterpret_cast<float *>(sh.txy), *Z = reinterpret_cast<float *>(sh.tz);
     const int q = lane >> 1, hh = lane & 1;
     X[4 * q + hh] = valid ? -x.x : 0.f;
     X[4 * q + 2 + hh] = valid ? -x.y : 0.f;
     Z[2 * q + hh] = valid ? -x.z : 0.f;
   }
-  int *pa = sh.pa[w];
-  unsigned *pmk = sh.pm[w];
   int sp = 1, np = 0, nf = 0, ng = 0, nn = 0;
   __syncwarp();
   tick<Count>(cnt, 8, t, lane);
@@ -487,181 +548,200 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
     if (sp > kWalkDrain)
     { // drain: each target walks the top range on its own
       sp--;
-      const int a = ia[sp], e = ie[sp];
+      const int2 r = ie[sp];
       const unsigned m = im[sp];
       __syncwarp();
       if (m & lanebit)
-        walk_range<Wrap>(T, a, e, x.x, x.y, x.z, K, h2, sum, comp, cnt);
+        walk_range<Wrap>(T, r.x, r.y, x.x, x.y, x.z, K, h2, sum, comp, cnt);
       if (Count && lane == 0)
         cnt.v[7]++;
       tick<Count>(cnt, 14, t, lane);
       continue;
     }
-    bool act, cell = false, near = true;
-    int a = 0, e = 0;
-    unsigned m = 0u, A = 0u, O = 0u;
-    float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (np >= kWarp || sp == 0)
-    { // resolve up to 32 pending cells, one per lane, each against every target
-      const int k = min(np, kWarp);
-      act = lane < k;
+    // Every lane reads a node (lanes past the last one read the last again,
+    // with no targets), so the step has no branches but its two kinds.
+    const bool resolve = np >= kWarp || sp == 0;
+    const int k = min(resolve ? np : sp, kWarp);
+    int a, e = 0;
+    unsigned m;
+    if (resolve)
+    { // pending cells, one per lane, each against every target
+      const int2 q = pend[np - k + min(lane, k - 1)];
+      a = q.x;
+      m = lane < k ? (unsigned)q.y : 0u;
+      np -= k;
       if (Count && lane == 0)
         cnt.v[3]++;
-      if (act)
-      {
-        a = pa[np - k + lane];
-        m = pmk[np - k + lane];
-      }
-      np -= k;
-      __syncwarp();
-      if (act)
-      {
-        na = __ldg(&T[a]);
-        nb = __ldg(&T[a + 1]);
-        cell = true;
-        e = __float_as_int(nb.y); // the cell's siblings are on the stack already
-        if (!Wrap)
-          near = box_gap2(lo, hi, na.x, na.y, na.z) < h2;
-        O = opens_mask<Wrap>(sh.txy[w], sh.tz[w], na.x, na.y, na.z,
-                             __uint_as_float(__float_as_uint(na.w) & 0x7fffffffu), nb.z, m, K);
-        A = m & ~O;
-      }
-      tick<Count>(cnt, 9, t, lane);
     }
     else
     { // the first nodes of up to 32 ranges, one per lane
-      const int k = min(sp, kWarp);
-      const int base = sp - k;
-      act = lane < k;
+      sp -= k;
+      const int at = sp + min(lane, k - 1);
+      const int2 r = ie[at];
+      a = r.x;
+      e = r.y;
+      m = lane < k ? im[at] : 0u;
       if (Count && lane == 0)
       {
         cnt.v[1]++;
         cnt.v[2] += k;
       }
-      if (act)
+    }
+    __syncwarp();
+    float4 na = __ldg(&T[a]);
+    const float4 nb = __ldg(&T[a + 1]); // a cell's mass, skip and side length (the tree has a padding slot)
+    const bool cell = slot_is_cell(na.w);
+    const float crit = __uint_as_float(__float_as_uint(na.w) & 0x7fffffffu);
+    const float ox = na.x, oy = na.y, oz = na.z; // the node's own centre
+    bool near = true;
+    unsigned A, O, flags = 0u;
+    float near2 = 0.f, far2 = 0.f;
+    if (Wrap)
+    { // the node, and the box, as the targets see each other
+      float wl[3] = {lo[0], lo[1], lo[2]}, wh[3] = {hi[0], hi[1], hi[2]};
+      na.x = wrap_axis(na.x, lo[0], hi[0], 0, flags, K);
+      na.y = wrap_axis(na.y, lo[1], hi[1], 1, flags, K);
+      na.z = wrap_axis(na.z, lo[2], hi[2], 2, flags, K);
+      if (flags & kMixed)
       {
-        a = ia[base + lane];
-        e = ie[base + lane];
-        m = im[base + lane];
+        na.x = ox;
+        na.y = oy;
+        na.z = oz;
       }
-      sp = base;
-      __syncwarp();
-      int cls = 0; // 0: every target accepts, 1: every target opens, 2: each target decides
-      if (act)
+      else
       {
-        na = __ldg(&T[a]);
-        nb = __ldg(&T[a + 1]); // a cell's mass, skip and side length (the tree has a padding slot)
-        cell = slot_is_cell(na.w);
-        if (Wrap)
-          cls = cell ? 2 : 0;
-        else
-        {
-          const float rmin2 = box_gap2(lo, hi, na.x, na.y, na.z);
-          near = rmin2 < h2;
-          if (cell)
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          if (flags & (1u << d))
           {
-            const float crit = __uint_as_float(__float_as_uint(na.w) & 0x7fffffffu);
-            if (!(rmin2 > __fmul_rn(crit, kBandHi)))
-            {
-              const float G[3] = {fmaxf(fabsf(__fsub_rn(na.x, lo[0])), fabsf(__fsub_rn(na.x, hi[0]))),
-                                  fmaxf(fabsf(__fsub_rn(na.y, lo[1])), fabsf(__fsub_rn(na.y, hi[1]))),
-                                  fmaxf(fabsf(__fsub_rn(na.z, lo[2])), fabsf(__fsub_rn(na.z, hi[2])))};
-              cls = dist2(G[0], G[1], G[2]) < __fmul_rn(crit, kBandLo) ? 1 : 2;
-            }
+            wl[d] = __fsub_rn(lo[d], K.box);
+            wh[d] = __fsub_rn(hi[d], K.box);
           }
-        }
+        if (resolve)
+          box_dist2(wl, wh, na.x, na.y, na.z, near2, far2);
       }
-      A = cls == 0 ? m : 0u;
-      O = cls == 1 ? m : 0u;
-      // cells near the targets' opening distance wait for a batch of their own
-      const unsigned bp = __ballot_sync(full, act && cls == 2);
-      if (act && cls == 2)
-      {
-        const int at = np + __popc(bp & below);
-        pa[at] = a;
-        pmk[at] = m;
+    }
+    else
+    {
+      box_dist2(lo, hi, na.x, na.y, na.z, near2, far2);
+      near = near2 < h2s;
+    }
+    if (resolve)
+    {
+      e = __float_as_int(nb.y); // the cell's siblings are on the stack already
+      if (Wrap)
+      { // the box may decide for every target; else each does
+        O = 0u;
+        if (flags & kMixed)
+          O = opens_mask_each(sh.txy, sh.tz, ox, oy, oz, crit, nb.z, m, K);
+        else if (!(near2 > __fmul_rn(crit, kBandHi)))
+          O = far2 < __fmul_rn(crit, kBandLo)
+                ? m
+                : opens_mask<true>(sh.txy, sh.tz, na.x, na.y, na.z, crit, nb.z, m, flags, ox, oy, oz, K);
       }
+      else
+        O = opens_mask<false>(sh.txy, sh.tz, na.x, na.y, na.z, crit, nb.z, m, 0u, ox, oy, oz, K);
+      A = m & ~O;
+      tick<Count>(cnt, 9, t, lane);
+    }
+    else
+    {
+      // every target accepts it (a leaf, or the box beyond the opening
+      // distance), every target opens it, or each decides on its own: cells
+      // near the targets' opening distance wait for a batch of their own
+      const bool acc = !cell || (!Wrap && near2 > __fmul_rn(crit, kBandHi));
+      const bool opn = !Wrap && far2 < __fmul_rn(crit, kBandLo);
+      A = acc ? m : 0u;
+      O = !acc && opn ? m : 0u;
+      const bool wait = !acc && !opn && m != 0u;
+      const unsigned bp = __ballot_sync(full, wait);
+      if (wait)
+        pend[np + __popc(bp & below)] = make_int2(a, (int)m);
       np += __popc(bp);
       tick<Count>(cnt, 8, t, lane);
     }
-    const bool has_e = act && A != 0u;
     const bool to_near = Wrap || near, every = A == vmask;
-    const unsigned bg = __ballot_sync(full, has_e && !to_near && every),
-                   bf = __ballot_sync(full, has_e && !to_near && !every), bn = __ballot_sync(full, has_e && to_near);
-    if (has_e)
+    const unsigned be = __ballot_sync(full, A != 0u);
+    if (be)
     {
-      const float4 en = make_float4(na.x, na.y, na.z, cell ? nb.x : na.w);
-      if (to_near)
+      const unsigned bn = be & (Wrap ? full : __ballot_sync(full, near)),
+                     bg = Wrap ? 0u : be & ~bn & __ballot_sync(full, every), bf = be & ~bn & ~bg;
+      if (A != 0u)
       {
-        const int at = nn + __popc(bn & below);
-        nea[at] = en;
-        nmsk[at] = A;
+        const int at = to_near ? kNearAt + nn + __popc(bn & below)
+                               : (every ? ng + __popc(bg & below) : kFarAt + nf + __popc(bf & below));
+        entry_put(ea, eb, at, na.x, na.y, na.z, -(cell ? nb.x : na.w));
+        if (at >= kFarAt)
+          mask[at - kFarAt] = A;
+        if (Wrap)
+          mask[at - kNearAt] = flags;
+        if (Count)
+          cnt.v[0] += __popc(A);
       }
-      else if (every)
-        full_put(ga, gb, ng + __popc(bg & below), en.x, en.y, en.z, en.w);
-      else
-        far_put(fa, fb, fm, nf + __popc(bf & below), en.x, en.y, en.z, en.w, A);
-      if (Count)
-        cnt.v[0] += __popc(A);
+      if (Count && lane == 0)
+      {
+        cnt.v[4] += __popc(bg);
+        cnt.v[5] += __popc(bf);
+        cnt.v[6] += __popc(bn);
+      }
+      ng += __popc(bg);
+      nf += __popc(bf);
+      nn += __popc(bn);
     }
-    if (Count && lane == 0)
-    {
-      cnt.v[4] += __popc(bg);
-      cnt.v[5] += __popc(bf);
-      cnt.v[6] += __popc(bn);
-    }
-    ng += __popc(bg);
-    nf += __popc(bf);
-    nn += __popc(bn);
     // the rest of each range, then the children of opened cells (popped first: depth first)
     const int next = cell ? __float_as_int(nb.y) : a + 1;
-    const bool has_sib = act && next < e, has_kid = act && O != 0u;
+    const bool has_sib = m != 0u && next < e, has_kid = O != 0u;
     const unsigned bs = __ballot_sync(full, has_sib), bk = __ballot_sync(full, has_kid);
     if (has_sib)
     {
       const int at = sp + __popc(bs & below);
-      ia[at] = next;
-      ie[at] = e;
+      ie[at] = make_int2(next, e);
       im[at] = m;
     }
     sp += __popc(bs);
     if (has_kid)
     {
       const int at = sp + __popc(bk & below);
-      ia[at] = a + 2;
-      ie[at] = next;
+      ie[at] = make_int2(a + 2, next);
       im[at] = O;
     }
     sp += __popc(bk);
     __syncwarp();
     tick<Count>(cnt, 10, t, lane);
-    if (ng > kWalkFull - kFlushMargin)
+    if (!Wrap && ng > kWalkFull - kFlushMargin)
     {
-      eval_full(ga, gb, pad8_full(ga, gb, ng, lane), x.x, x.y, x.z, sum, comp);
+      eval_far<false>(ea, eb, nullptr, pad8(ea, eb, mask, 0, ng, lane), lanebit, x.x, x.y, x.z, sum, comp);
       ng = 0;
       __syncwarp();
       tick<Count>(cnt, 11, t, lane);
     }
-    if (nf > kWalkFar - kFlushMargin)
+    if (!Wrap && nf > kWalkFar - kFlushMargin)
     {
-      eval_far(fa, fb, fm, pad8_far(fa, fb, fm, nf, lane), lanebit, x.x, x.y, x.z, sum, comp);
+      eval_far<true>(ea + kFarAt / 2, eb + kFarAt / 2, mask, pad8(ea, eb, mask, kFarAt, nf, lane), lanebit, x.x, x.y,
+                     x.z, sum, comp);
       nf = 0;
       __syncwarp();
       tick<Count>(cnt, 12, t, lane);
     }
     if (nn > kWalkNear - kFlushMargin)
     {
-      eval_near<Wrap>(nea, nmsk, pad8(nea, nmsk, nn, lane), lanebit, x.x, x.y, x.z, K, h2, sum, comp);
+      eval_near<Wrap>(ea + kNearAt / 2, eb + kNearAt / 2, mask + kWalkFar, mask, pad8(ea, eb, mask, kNearAt, nn, lane),
+                      lanebit, x.x, x.y, x.z, K, h2, h2s, sum, comp);
       nn = 0;
       __syncwarp();
       tick<Count>(cnt, 13, t, lane);
     }
   }
-  eval_full(ga, gb, pad8_full(ga, gb, ng, lane), x.x, x.y, x.z, sum, comp);
-  tick<Count>(cnt, 11, t, lane);
-  eval_far(fa, fb, fm, pad8_far(fa, fb, fm, nf, lane), lanebit, x.x, x.y, x.z, sum, comp);
-  tick<Count>(cnt, 12, t, lane);
-  eval_near<Wrap>(nea, nmsk, pad8(nea, nmsk, nn, lane), lanebit, x.x, x.y, x.z, K, h2, sum, comp);
+  if (!Wrap)
+  {
+    eval_far<false>(ea, eb, nullptr, pad8(ea, eb, mask, 0, ng, lane), lanebit, x.x, x.y, x.z, sum, comp);
+    tick<Count>(cnt, 11, t, lane);
+    eval_far<true>(ea + kFarAt / 2, eb + kFarAt / 2, mask, pad8(ea, eb, mask, kFarAt, nf, lane), lanebit, x.x, x.y, x.z,
+                   sum, comp);
+    tick<Count>(cnt, 12, t, lane);
+  }
+  eval_near<Wrap>(ea + kNearAt / 2, eb + kNearAt / 2, mask + kWalkFar, mask, pad8(ea, eb, mask, kNearAt, nn, lane),
+                  lanebit, x.x, x.y, x.z, K, h2, h2s, sum, comp);
   __syncwarp();
   tick<Count>(cnt, 13, t, lane);
   t = t_all;
@@ -674,8 +754,8 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
 // reference: a target that is a tree source starts from +m/soft, cancelling
 // its own leaf, src/gravity_tree.cpp:98-101).
 template <bool Count>
-__device__ __forceinline__ void walk_chunk(const DevState &D, const KParams &K, int c, int lane, WalkShared &sh,
-                                           int w, WalkCount &cnt)
+__device__ __forceinline__ void walk_chunk(const DevState &D, const KParams &K, int c, int lane, WalkWarp &sh,
+                                           WalkCount &cnt)
 {
   const int s = find_segment_warp(D.chunk_off, D.S, c); // c is the same on every lane
   const int t = (c - D.chunk_off[s]) * kWarp + lane;
@@ -697,9 +777,9 @@ __device__ __forceinline__ void walk_chunk(const DevState &D, const KParams &K, 
   }
   const int root = D.src_off[s] + 2 * D.X[D.src_off[s]];
   if (D.wrap[s])
-    walk_group<true, Count>(D, K, s, root, lane, valid, p, x, self, sh, w, cnt);
+    walk_group<true, Count>(D, K, s, root, lane, valid, p, x, self, sh, cnt);
   else
-    walk_group<false, Count>(D, K, s, root, lane, valid, p, x, self, sh, w, cnt);
+    walk_group<false, Count>(D, K, s, root, lane, valid, p, x, self, sh, cnt);
 }
 
 // With walk counters, the chunks (key order) are split into `nranges`
@@ -716,8 +796,9 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
 #endif
   k_walk(DevState D, KParams K, int total_chunks, int nranges)
 {
-  __shared__ WalkShared sh;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __shared__ WalkWarp shared[kWalkWarps];
+  const int lane = threadIdx.x & 31;
+  WalkWarp &sh = shared[threadIdx.x >> 5];
   WalkCount cnt = {};
   if (D.walk_ctr)
   {
@@ -738,7 +819,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
         tries++;
         continue;
       }
-      walk_chunk<Count>(D, K, (int)c, lane, sh, w, cnt);
+      walk_chunk<Count>(D, K, (int)c, lane, sh, cnt);
     }
   }
   else
@@ -746,7 +827,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int c = warp_global; c < total_chunks; c += nwarps)
-      walk_chunk<Count>(D, K, c, lane, sh, w, cnt);
+      walk_chunk<Count>(D, K, c, lane, sh, cnt);
   }
   if (Count)
     for (int q = 0; q < kWalkCounters; q++)
