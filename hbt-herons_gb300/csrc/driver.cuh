@@ -16,6 +16,8 @@
 //   int *level_counts()                          2 kLevels ints
 //   float4 *tree_slots(long long slots)          tree storage (may throw when too large)
 //   void mark(int phase)                         phase boundary for timing (may be a no-op)
+//   static constexpr bool kTeams                 whether it has working buffers for k_settle (else lock step to the end)
+//   void settle_buffers(SettleArgs &, int S, int grid)  those buffers, for a grid's team of that many blocks
 #pragma once
 
 #include <algorithm>
@@ -25,6 +27,7 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "primitives.cuh"
+#include "settle.cuh"
 #include "walk.cuh"
 
 namespace hbtg
@@ -56,6 +59,8 @@ struct IterationDriver
   int64_t tree_nodes = 0;
   int64_t host_syncs = 0; // stream synchronisations for host reads of device totals
   int global_iter = 0;
+  int settle_from = -1; // lock-step iterations before the first k_settle of the call (-1: none)
+  SettleArgs settle_args{};
 
   IterationDriver(Mem &m, cudaStream_t s) : mem(m), st(s)
   {
@@ -283,6 +288,68 @@ struct IterationDriver
     check();
   }
 
+  // The active subhaloes that fit a team run to their end there.
+  void settle(long long live)
+  {
+    SettleArgs &A = settle_args;
+    mem.settle_buffers(A, S, live > kSettleMid ? settle_grid() : 0);
+    if (settle_from < 0)
+    {
+      settle_from = global_iter;
+      mem.check(cudaMemsetAsync(A.cells, 0, sizeof(*A.cells), st));
+      mem.check(cudaMemsetAsync(A.most, 0, sizeof(*A.most), st));
+    }
+    mem.check(cudaMemsetAsync(A.count, 0, kSettleClasses * sizeof(int), st));
+    k_settle_pick<<<grid_for(S, 256), 256, 0, st>>>(D, K, A);
+    launch_settle<1>(std::min(S, kSettleTeams1));
+    launch_settle<kSettleCluster>(std::min(S, kSettleTeams8) * kSettleCluster);
+    if (live > kSettleMid) // else no subhalo is that large
+    {
+      launch_settle<kGrid>(settle_grid());
+      launches++;
+    }
+    launches += 3;
+    check();
+    mem.mark(1);
+  }
+
+  // Blocks of the grid's team: all must be resident.
+  int settle_grid()
+  {
+    const int smem = (int)sizeof(SettleShared);
+    int per_sm = 0;
+    mem.check(cudaFuncSetAttribute(k_settle<kGrid>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    mem.check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_settle<kGrid>, kSettleThreads, (size_t)smem));
+    return std::min(kSettleMaxBlocks, sm_count * std::max(1, std::min(per_sm, kSettleGridPerSm)));
+  }
+
+  template <int C>
+  void launch_settle(int blocks)
+  {
+    const int smem = (int)sizeof(SettleShared);
+    mem.check(cudaFuncSetAttribute(k_settle<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kSettleThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (C == kGrid)
+    {
+      attr[0].id = cudaLaunchAttributeCooperative;
+      attr[0].val.cooperative = 1;
+    }
+    else
+    {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = C;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = C != 1 ? 1 : 0;
+    mem.check(cudaLaunchKernelEx(&cfg, k_settle<C>, D, K, settle_args));
+  }
+
   void run()
   {
     mem.mark(-1);
@@ -294,8 +361,15 @@ struct IterationDriver
   void iterate()
   {
     const unsigned sb = grid_for(S + 1, 256);
+    // Particles that the next iteration's bound sets can hold.  Once they are
+    // at most kComSmall, the subhaloes that fit go to teams (settle.cuh): not
+    // earlier, because only there do both add the same centre-of-mass terms.
+    long long live = D.N;
     for (;;)
     {
+      if constexpr (Mem::kTeams)
+        if (live <= kComSmall && live > 0 && !K.count_interactions)
+          settle(live);
       k_plan<<<sb, 256, 0, st>>>(D, K);
       launches++;
       check();
@@ -340,6 +414,7 @@ struct IterationDriver
         int tb[4];
         scan_counts4(D.tail_cnt, D.tail_off, D.fin_cnt, D.fin_off, nullptr, nullptr, nullptr, nullptr, S, tb);
         const int tail_total = tb[0], bound_total = tb[1];
+        live = bound_total;
         if (tail_total > 0)
         {
           k_energy_keys<<<grid_for(tail_total, 256), 256, 0, st>>>(D, D.tail_off, tail_total, 0);

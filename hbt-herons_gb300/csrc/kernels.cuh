@@ -364,6 +364,38 @@ __global__ void __launch_bounds__(256) k_bbox(DevState D, int total)
   }
 }
 
+// Fast-descent constants of a root cube of side len about the box [lo, hi]:
+// kp[0..2] + kp[3..5] its origin per axis as a float pair, kp[6] = 2^21 /
+// side, kp[7] the number of levels that must match the reference exactly
+// (cells not smaller than TreeNodeResolution, plus one), kp[8] the halvings
+// until the side drops below TreeNodeResolution, kp[11] the side.
+__device__ __forceinline__ void root_axis(double lo, double hi, double len, float *kp, int d)
+{
+  const double o = 0.5 * (hi + lo) - 0.5 * len;
+  kp[d] = (float)o;
+  kp[3 + d] = (float)(o - (double)(float)o);
+}
+__device__ __forceinline__ void root_levels(double len, const KParams &K, float *kp)
+{
+  kp[6] = len > 0. ? (float)(2097152.0 / len) : 0.f;
+  int exact_levels = 21;
+  if (K.res > 0.f && len > 0.)
+  {
+    const double lv = floor(log2(len / (double)K.res)) + 2.;
+    exact_levels = lv < 1. ? 1 : (lv > 21. ? 21 : (int)lv);
+  }
+  kp[7] = __int_as_float(exact_levels);
+}
+// A cell at level L has side len * 2^-min(L, kstar) (src/gravity_tree.cpp:38-42).
+__device__ __forceinline__ void root_sides(double len, const KParams &K, float *kp)
+{
+  int kstar = 0;
+  for (double l = len; l >= (double)K.res && kstar < 1000; l *= 0.5)
+    kstar++;
+  kp[8] = __int_as_float(kstar);
+  kp[11] = (float)len;
+}
+
 // Root cube (src/oct_tree.tpp:44-65): centre of the box, side = largest extent.
 // Built for every subhalo with sources: the active ones, and the converged
 // ones whose most-bound prefix gets its own tree (RefineBindingEnergyOrder).
@@ -385,31 +417,11 @@ __global__ void k_root(DevState D, KParams K)
   for (int d = 0; d < 3; d++)
     D.root[4 * s + d] = 0.5 * (hi[d] + lo[d]);
   D.root[4 * s + 3] = len;
-  // fast-descent constants: origin of the root cube per axis as a float pair,
-  // 2^21 / side, and the number of levels that must match the reference
-  // exactly (cells not smaller than TreeNodeResolution, plus one)
   float *kp = D.keyp + 12 * s;
   for (int d = 0; d < 3; d++)
-  {
-    const double o = 0.5 * (hi[d] + lo[d]) - 0.5 * len;
-    kp[d] = (float)o;
-    kp[3 + d] = (float)(o - (double)(float)o);
-  }
-  kp[6] = len > 0. ? (float)(2097152.0 / len) : 0.f;
-  int exact_levels = 21;
-  if (K.res > 0.f && len > 0.)
-  {
-    const double lv = floor(log2(len / (double)K.res)) + 2.;
-    exact_levels = lv < 1. ? 1 : (lv > 21. ? 21 : (int)lv);
-  }
-  kp[7] = __int_as_float(exact_levels);
-  // halvings until the side drops below TreeNodeResolution: a cell at level L
-  // has side len * 2^-min(L, kstar) (src/gravity_tree.cpp:38-42)
-  int kstar = 0;
-  for (double l = len; l >= (double)K.res && kstar < 1000; l *= 0.5)
-    kstar++;
-  kp[8] = __int_as_float(kstar);
-  kp[11] = (float)len;
+    root_axis(lo[d], hi[d], len, kp, d);
+  root_levels(len, K, kp);
+  root_sides(len, K, kp);
   // first iteration: the sources are every particle (a warm start decides the
   // wrap from every particle before it starts)
   if (D.state[s] == kActive && D.iter[s] == 1 && !D.corr[s] && !(D.warm && D.warm[s] == 1))
@@ -517,7 +529,7 @@ __global__ void k_keys(DevState D, int total)
   }
 }
 
-// Items the fast descent could not decide.  Per axis the exact-level slab
+// Key of a particle that the fast descent could not decide.  Per axis the exact-level slab
 // index (slabs of width w = side 2^-lv, cells left-open, right-closed) lies
 // within one of the float estimate's, so two exact comparisons in double
 // settle it: x > o + m w with o the root cube's origin, the same dyadic
@@ -525,6 +537,40 @@ __global__ void k_keys(DevState D, int total)
 // without rounding.  The digits below the exact levels follow the float
 // estimate, kept inside the decided cell.  A non-finite estimate takes the
 // reference's descent level by level.
+__device__ __noinline__ unsigned long long descent_key_exact(float4 x, const float *kp, const double *r)
+{
+  const int lv = __float_as_int(kp[7]);
+  const int low = 21 - lv;
+  const float xs[3] = {x.x, x.y, x.z};
+  const double w = r[3] * __hiloint2double((1023 - lv) << 20, 0); // side 2^-lv, exact
+  const float inv_unit = __int_as_float((127 - low) << 23);       // 2^-low
+  const unsigned top = (1u << lv) - 1u;
+  unsigned long long key = 0;
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+  {
+    const float t = __fmul_rn(__fsub_rn(__fsub_rn(xs[d], kp[d]), kp[3 + d]), kp[6]);
+    if (!(t > -1e30f && t < 1e30f))
+      return descent_key(x, r);
+    const float tl = floorf(__fmul_rn(t, inv_unit));
+    const int m0 = (int)fminf(fmaxf(tl, -1.f), (float)top + 1.f);
+    const double dx = (double)xs[d] - (r[d] - 0.5 * r[3]); // x - o
+    int k = m0 - 1; // sign of dx - m w from one fused rounding: exact
+    if (fma(-(double)m0, w, dx) > 0.)
+      k = (fma(-(double)(m0 + 1), w, dx) > 0.) ? m0 + 1 : m0;
+    k = k < 0 ? 0 : (k > (int)top ? (int)top : k);
+    // digits below the exact levels: the float slab index, clamped into slab k
+    float c = floorf(t);
+    c = c < 0.f ? 0.f : (c > 2097151.f ? 2097151.f : c);
+    unsigned c21 = __float2uint_rz(c);
+    const unsigned lo21 = (unsigned)k << low, hi21 = lo21 | ((1u << low) - 1u);
+    c21 = c21 < lo21 ? lo21 : (c21 > hi21 ? hi21 : c21);
+    key |= spread3((unsigned long long)c21) << d;
+  }
+  return key;
+}
+
+// The items that k_keys left to the exact descent.
 __global__ void k_keys_fallback(DevState D)
 {
   const int n = *D.fb_count;
@@ -533,44 +579,7 @@ __global__ void k_keys_fallback(DevState D)
     const int j = D.fb_list[i];
     const int p = (int)D.val[j];
     const int s = D.seg_of[p];
-    const float *kp = D.keyp + 12 * s;
-    const double *r = D.root + 4 * s;
-    const int lv = __float_as_int(kp[7]);
-    const int low = 21 - lv;
-    const float4 x = D.pm[p];
-    const float xs[3] = {x.x, x.y, x.z};
-    const double w = r[3] * __hiloint2double((1023 - lv) << 20, 0); // side 2^-lv, exact
-    const float inv_unit = __int_as_float((127 - low) << 23);       // 2^-low
-    const unsigned top = (1u << lv) - 1u;
-    unsigned long long key = 0;
-    bool finite = true;
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-    {
-      const float t = __fmul_rn(__fsub_rn(__fsub_rn(xs[d], kp[d]), kp[3 + d]), kp[6]);
-      if (!(t > -1e30f && t < 1e30f))
-      {
-        finite = false;
-        break;
-      }
-      const float tl = floorf(__fmul_rn(t, inv_unit));
-      const int m0 = (int)fminf(fmaxf(tl, -1.f), (float)top + 1.f);
-      const double dx = (double)xs[d] - (r[d] - 0.5 * r[3]); // x - o
-      int k = m0 - 1; // sign of dx - m w from one fused rounding: exact
-      if (fma(-(double)m0, w, dx) > 0.)
-        k = (fma(-(double)(m0 + 1), w, dx) > 0.) ? m0 + 1 : m0;
-      k = k < 0 ? 0 : (k > (int)top ? (int)top : k);
-      // digits below the exact levels: the float slab index, clamped into slab k
-      float c = floorf(t);
-      c = c < 0.f ? 0.f : (c > 2097151.f ? 2097151.f : c);
-      unsigned c21 = __float2uint_rz(c);
-      const unsigned lo21 = (unsigned)k << low, hi21 = lo21 | ((1u << low) - 1u);
-      c21 = c21 < lo21 ? lo21 : (c21 > hi21 ? hi21 : c21);
-      key |= spread3((unsigned long long)c21) << d;
-    }
-    if (!finite)
-      key = descent_key(x, r);
-    D.key[j] = key;
+    D.key[j] = descent_key_exact(D.pm[p], D.keyp + 12 * s, D.root + 4 * s);
   }
 }
 
@@ -807,6 +816,16 @@ __device__ __forceinline__ void ll_to_float2(long long v, float &hi, float &lo)
   lo = v < 0 ? -l : l;
 }
 
+// The two slots of a cell at level L of a root cube with constants kp whose
+// subtree ends before slot `skip`; its mass and centre come later.
+__device__ __forceinline__ void put_cell(float4 *slot, const float *kp, int L, int skip, const KParams &K)
+{
+  const float lenf = ldexpf(kp[11], -min(L, __float_as_int(kp[8])));
+  const float crit = __fdiv_rn(__fmul_rn(lenf, lenf), K.theta2);
+  slot[0] = make_float4(0.f, 0.f, 0.f, __uint_as_float(__float_as_uint(crit) | 0x80000000u));
+  slot[1] = make_float4(0.f, __int_as_float(skip), lenf, 0.f);
+}
+
 // One cell: item j's cell at level L (slot `slot`), in segment s ending at
 // seg_end.  Its last item b is found by galloping forward from j over the
 // keys; that gives the slot after its subtree (its skip).  The cell's side
@@ -846,13 +865,7 @@ __device__ __forceinline__ void emit_cell(const DevState &D, const KParams &K, i
     }
     b = a;
   }
-  const float *kp = D.keyp + 12 * s;
-  const int kstar = __float_as_int(kp[8]);
-  const float lenf = ldexpf(kp[11], -min(L, kstar));
-  const float crit = __fdiv_rn(__fmul_rn(lenf, lenf), K.theta2);
-  const int skip = b + 2 * D.X[b] + 2 * D.cnt[b] + 1;
-  D.nodes[slot] = make_float4(0.f, 0.f, 0.f, __uint_as_float(__float_as_uint(crit) | 0x80000000u));
-  D.nodes[slot + 1] = make_float4(0.f, __int_as_float(skip), lenf, 0.f);
+  put_cell(D.nodes + slot, D.keyp + 12 * s, L, b + 2 * D.X[b] + 2 * D.cnt[b] + 1, K);
 }
 
 // Writes the tree slots in preorder.  Slot index: cell (j, level lo+t) =
@@ -942,20 +955,20 @@ __global__ void k_tree_emit(DevState D, KParams K, int total)
 // rounding, so a cell's centre carries its children's roundings as in the
 // reference.
 // The multipoles of the cell at `slot` from its children.
-__device__ __forceinline__ void cell_moments(const DevState &D, int slot)
+__device__ __forceinline__ void cell_moments(float4 *nodes, int slot)
 {
-  const int end = __float_as_int(D.nodes[slot + 1].y);
+  const int end = __float_as_int(nodes[slot + 1].y);
   double M = 0., X = 0., Y = 0., Z = 0.;
   float fx = 0.f, fy = 0.f, fz = 0.f; // first child's position (a massless cell)
   int ch = slot + 2;
   while (ch < end)
   {
-    const float4 a = D.nodes[ch];
+    const float4 a = nodes[ch];
     float m;
     int nx;
     if (slot_is_cell(a.w))
     {
-      const float4 b = D.nodes[ch + 1];
+      const float4 b = nodes[ch + 1];
       m = b.x;
       nx = __float_as_int(b.y);
     }
@@ -977,7 +990,7 @@ __device__ __forceinline__ void cell_moments(const DevState &D, int slot)
     Z = __fma_rn((double)a.z, md, Z);
     ch = max(nx, ch + 1); // strictly increasing
   }
-  float *cs = reinterpret_cast<float *>(&D.nodes[slot]);
+  float *cs = reinterpret_cast<float *>(&nodes[slot]);
   if (M > 0.)
   {
     cs[0] = __double2float_rn(__ddiv_rn(X, M));
@@ -990,7 +1003,7 @@ __device__ __forceinline__ void cell_moments(const DevState &D, int slot)
     cs[1] = fy;
     cs[2] = fz;
   }
-  reinterpret_cast<float *>(&D.nodes[slot + 1])[0] = __double2float_rn(M);
+  reinterpret_cast<float *>(&nodes[slot + 1])[0] = __double2float_rn(M);
 }
 
 // The cells of level L (deepest level first, one launch per level).
@@ -1001,7 +1014,7 @@ __global__ void k_tree_moments(DevState D, int L)
     off += D.lvl[l];
   const int n = D.lvl[L];
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-    cell_moments(D, D.cell_list[off + c]);
+    cell_moments(D.nodes, D.cell_list[off + c]);
 }
 
 // Geometric trees (neighbour searches): each cell's bounding box of its
@@ -1101,6 +1114,30 @@ __device__ __forceinline__ float norm2_rn(const float *d)
   return __fadd_rn(__fadd_rn(__fmul_rn(d[0], d[0]), __fmul_rn(d[1], d[1])), __fmul_rn(d[2], d[2]));
 }
 
+// Binding energy of a particle at x, v in the frame (rp, rv) with tree
+// potential pot (src/gravity_tree.cpp:168-178, src/subhalo_unbind.cpp:563-580).
+__device__ __forceinline__ float binding_energy(float4 x, float4 v, float pot, const float *rp, const float *rv,
+                                                const KParams &K)
+{
+  float dv[3];
+  rel_vel(make_float3(x.x, x.y, x.z), make_float3(v.x, v.y, v.z), rp, rv, K, dv);
+  const float e = __fadd_rn(__fmul_rn(0.5f, norm2_rn(dv)), pot);
+  return K.thermal ? __fadd_rn(e, v.w) : e;
+}
+
+// Its energy e after the frame moved from (op, ov) to (rp, rv) and the
+// removed particles, of potential pot, left (src/subhalo_unbind.cpp:583-616).
+__device__ __forceinline__ float corrected_energy(float e, float4 x, float4 v, float pot, const float *op,
+                                                  const float *ov, const float *rp, const float *rv, const KParams &K)
+{
+  float dV[3], dv[3];
+  rel_vel(make_float3(op[0], op[1], op[2]), make_float3(ov[0], ov[1], ov[2]), rp, rv, K, dV);
+  const float dK = __fmul_rn(0.5f, norm2_rn(dV)); // halving is exact
+  rel_vel(make_float3(x.x, x.y, x.z), make_float3(v.x, v.y, v.z), op, ov, K, dv);
+  const float dot = __fadd_rn(__fadd_rn(__fmul_rn(dv[0], dV[0]), __fmul_rn(dv[1], dV[1])), __fmul_rn(dv[2], dV[2]));
+  return __fadd_rn(e, __fsub_rn(__fadd_rn(dot, dK), pot));
+}
+
 __global__ void k_energy(DevState D, KParams K, int total)
 {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1110,28 +1147,9 @@ __global__ void k_energy(DevState D, KParams K, int total)
   const int k = j - D.part_off[s];
   const int p = D.ord[D.off[s] + k];
   const float4 x = D.pm[p], v = D.vu[p];
-  const float3 x3 = make_float3(x.x, x.y, x.z), v3 = make_float3(v.x, v.y, v.z);
-  if (!D.corr[s])
-  {
-    float dv[3];
-    rel_vel(x3, v3, D.ref_pos + 3 * s, D.ref_vel + 3 * s, K, dv);
-    float e = __fadd_rn(__fmul_rn(0.5f, norm2_rn(dv)), D.pot[p]);
-    if (K.thermal)
-      e = __fadd_rn(e, v.w);
-    D.Ep[p] = e;
-  }
-  else
-  {
-    float dV[3], ov[3];
-    const float op[3] = {D.old_pos[3 * s], D.old_pos[3 * s + 1], D.old_pos[3 * s + 2]};
-    const float ovl[3] = {D.old_vel[3 * s], D.old_vel[3 * s + 1], D.old_vel[3 * s + 2]};
-    rel_vel(make_float3(op[0], op[1], op[2]), make_float3(ovl[0], ovl[1], ovl[2]), D.ref_pos + 3 * s,
-            D.ref_vel + 3 * s, K, dV);
-    const float dK = __fmul_rn(0.5f, norm2_rn(dV)); // halving is exact
-    rel_vel(x3, v3, op, ovl, K, ov);
-    const float dot = __fadd_rn(__fadd_rn(__fmul_rn(ov[0], dV[0]), __fmul_rn(ov[1], dV[1])), __fmul_rn(ov[2], dV[2]));
-    D.Ep[p] = __fadd_rn(D.Ep[p], __fsub_rn(__fadd_rn(dot, dK), D.pot[p]));
-  }
+  const float *rp = D.ref_pos + 3 * s, *rv = D.ref_vel + 3 * s;
+  D.Ep[p] = D.corr[s] ? corrected_energy(D.Ep[p], x, v, D.pot[p], D.old_pos + 3 * s, D.old_vel + 3 * s, rp, rv, K)
+                      : binding_energy(x, v, D.pot[p], rp, rv, K);
 }
 
 __global__ void k_part_flags(DevState D, int total)
@@ -1377,6 +1395,18 @@ struct KahanF
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
+// Mass-weighted coordinate of a particle in the centre-of-mass sums, about the
+// bound set's first particle at o.
+__device__ __forceinline__ float com_offset(float x, float o, float m, const KParams &K)
+{
+  if (!K.periodic)
+    return __fmul_rn(x, m);
+  const float df = x - o;
+  if (fabsf(df) < 0.25f * K.half) // no wrap possible; x - o is exact or nearly so
+    return __fmul_rn(df, m);
+  return (float)(nearest_d((double)x - (double)o, K.half, K.box) * m);
+}
+
 // Centre-of-mass sums over the bound set, wrapped about its first particle
 // (src/subhalo_unbind.cpp:151-198).  Each thread sums 16 consecutive items
 // with compensated float partials (FP64 is scarce on this GPU); the partials
@@ -1420,18 +1450,7 @@ __global__ void k_com(DevState D, KParams K, int total)
       const float xs[3] = {x.x, x.y, x.z}, os[3] = {o.x, o.y, o.z};
 #pragma unroll
       for (int d = 0; d < 3; d++)
-      {
-        if (K.periodic)
-        {
-          const float df = xs[d] - os[d];
-          if (fabsf(df) < 0.25f * K.half) // no wrap possible; x - o is exact or nearly so
-            acc[1 + d].add(__fmul_rn(df, m));
-          else
-            acc[1 + d].add((float)(nearest_d((double)xs[d] - (double)os[d], K.half, K.box) * m));
-        }
-        else
-          acc[1 + d].add(__fmul_rn(xs[d], m));
-      }
+        acc[1 + d].add(com_offset(xs[d], os[d], m, K));
       acc[4].add(__fmul_rn(v.x, m));
       acc[5].add(__fmul_rn(v.y, m));
       acc[6].add(__fmul_rn(v.z, m));

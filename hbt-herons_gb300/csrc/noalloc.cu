@@ -144,6 +144,7 @@ inline unsigned nblocks(long long n, int threads)
 // of the static reserve; a request beyond its size fails the call.
 struct StaticMem
 {
+  static constexpr bool kTeams = false;
   int *scan_scr = nullptr, *table = nullptr;
   int *cells = nullptr, *lvl = nullptr;
   float4 *slots = nullptr;

@@ -166,6 +166,7 @@ enum Slot
   S_PR_OFF, S_PR_CNT, S_PR_FIN, S_PR_RR, S_PR_MM, S_PR_K, S_PR_V, S_PR_KA, S_PR_VA, S_PR_MC, S_PR_VK, S_PR_SO,
   S_PR_SH, S_PR_SCR, S_PR_POS, S_PR_MASS, S_PR_ORD, S_PR_NB, S_PR_MBND, S_PR_MBP, S_PR_OUTF, S_PR_OUTI, S_PR_OUTL,
   S_RE_OFF, S_RE_SG, S_RE_GP, S_RE_FL, S_RE_RK, S_RE_TG, S_RE_TS, S_RE_GO, S_RE_POS, S_RE_TY, S_RE_DEST,
+  S_SET_LIST, S_SET_NODES, S_SET_KEY, S_SET_VAL, S_SET_XCH, S_SET_TOT,
   S_RE_QK, S_RE_QKA, S_RE_QV, S_RE_QVA,
   S_NUM
 };
@@ -356,6 +357,22 @@ struct PoolMem
     if (slots >= (1LL << 31) - 64)
       throw NoMem{};
     return H->pool.get<float4>(S_NODES, (size_t)slots);
+  }
+  static constexpr bool kTeams = true;
+  void settle_buffers(SettleArgs &A, int S, int grid)
+  {
+    Pool &P = H->pool;
+    const size_t teams8 = (size_t)std::min(S, kSettleTeams8),
+                 blocks = std::max({(size_t)std::min(S, kSettleTeams1), teams8 * kSettleCluster, (size_t)grid});
+    A.list = P.get<int>(S_SET_LIST, kSettleClasses * (size_t)S);
+    A.nodes = P.get<float4>(S_SET_NODES, blocks * kSettleSlots);
+    A.skey = P.get<unsigned long long>(S_SET_KEY, teams8 * kSettleSrc);
+    A.sval = P.get<uint32_t>(S_SET_VAL, teams8 * kSettleSrc);
+    A.xch = P.get<double>(S_SET_XCH, 2 * 8 * std::max(teams8 * kSettleCluster, (size_t)grid));
+    unsigned long long *tot = P.get<unsigned long long>(S_SET_TOT, 2 + kSettleClasses);
+    A.cells = tot;
+    A.most = reinterpret_cast<int *>(tot + 1);
+    A.count = reinterpret_cast<int *>(tot + 2);
   }
   void mark(int phase)
   {
@@ -618,6 +635,13 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
   H->stats.walk_blocks_per_sm = R.walk_blocks_per_sm;
   H->stats.global_iterations = R.global_iter;
   H->stats.tree_nodes = R.tree_nodes;
+  if (R.settle_from >= 0)
+  { // the teams' share
+    unsigned long long tot[2] = {};
+    HBTG_CUDA(cudaMemcpy(tot, R.settle_args.cells, sizeof(tot), cudaMemcpyDeviceToHost));
+    H->stats.tree_nodes += (int64_t)tot[0];
+    H->stats.global_iterations = std::max<int64_t>(R.global_iter, R.settle_from + (int)(tot[1] & 0xffffffffu));
+  }
   if (H->count_interactions)
   {
     unsigned long long c[kWalkCounters] = {};

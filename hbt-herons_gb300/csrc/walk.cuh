@@ -465,21 +465,29 @@ __device__ __forceinline__ void eval_near(const float4 *ea, const float4 *eb, co
   }
 }
 
+// A tree slot; Fresh: the tree may have been written by this kernel, so not
+// through the read-only path.
+template <bool Fresh>
+__device__ __forceinline__ float4 tree_slot(const float4 *p)
+{
+  return Fresh ? __ldca(p) : __ldg(p);
+}
+
 // The reference's stackless walk of one range [a, e) of sibling subtrees for
 // one target (open: next slot; accept: interact and skip the subtree).
-template <bool Wrap>
-__device__ __forceinline__ void walk_range(const float4 *__restrict__ T, int a, int e, float tx, float ty, float tz,
+template <bool Wrap, bool Fresh>
+__device__ __forceinline__ void walk_range(const float4 *T, int a, int e, float tx, float ty, float tz,
                                            const KParams &K, float h2, float &sum, float &comp, WalkCount &cnt)
 {
   int idx = a;
   while (idx < e)
   {
-    const float4 n = __ldg(&T[idx]);
+    const float4 n = tree_slot<Fresh>(&T[idx]);
     float m;
     int next;
     if (slot_is_cell(n.w))
     {
-      const float4 b = __ldg(&T[idx + 1]);
+      const float4 b = tree_slot<Fresh>(&T[idx + 1]);
       const float crit = __uint_as_float(__float_as_uint(n.w) & 0x7fffffffu);
       if (target_opens<Wrap>(n.x, n.y, n.z, crit, b.z, tx, ty, tz, K))
       {
@@ -501,12 +509,13 @@ __device__ __forceinline__ void walk_range(const float4 *__restrict__ T, int a, 
   }
 }
 
-// Potentials of the (up to) 32 targets of chunk c.
-template <bool Wrap, bool Count>
-__device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, int s, int root, int lane, bool valid,
+// Potentials of (up to) 32 targets in the tree T with the given root slot: the
+// calling warp's lane holds target particle p at x (mass in w) with its self
+// term; valid = false: no target.
+template <bool Wrap, bool Count, bool Fresh>
+__device__ __forceinline__ void walk_group(const float4 *T, float *pot, const KParams &K, int root, int lane, bool valid,
                                            int p, float4 x, float self, WalkWarp &sh, WalkCount &cnt)
 {
-  const float4 *__restrict__ T = D.nodes;
   float4 *ea = sh.a, *eb = sh.b;
   unsigned *mask = sh.mask;
   int2 *ie = sh.ie, *pend = sh.pend;
@@ -529,7 +538,7 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
   float sum = valid ? self / K.soft : 0.f, comp = 0.f;
   if (lane == 0)
   {
-    ie[0] = make_int2(root, __float_as_int(__ldg(&T[root + 1]).y));
+    ie[0] = make_int2(root, __float_as_int(tree_slot<Fresh>(&T[root + 1]).y));
     im[0] = vmask;
   }
   // the targets, negated, in pairs (the pending cells' tests read them)
@@ -552,7 +561,7 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
       const unsigned m = im[sp];
       __syncwarp();
       if (m & lanebit)
-        walk_range<Wrap>(T, r.x, r.y, x.x, x.y, x.z, K, h2, sum, comp, cnt);
+        walk_range<Wrap, Fresh>(T, r.x, r.y, x.x, x.y, x.z, K, h2, sum, comp, cnt);
       if (Count && lane == 0)
         cnt.v[7]++;
       tick<Count>(cnt, 14, t, lane);
@@ -588,8 +597,8 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
       }
     }
     __syncwarp();
-    float4 na = __ldg(&T[a]);
-    const float4 nb = __ldg(&T[a + 1]); // a cell's mass, skip and side length (the tree has a padding slot)
+    float4 na = tree_slot<Fresh>(&T[a]);
+    const float4 nb = tree_slot<Fresh>(&T[a + 1]); // a cell's mass, skip and side length (the tree has a padding slot)
     const bool cell = slot_is_cell(na.w);
     const float crit = __uint_as_float(__float_as_uint(na.w) & 0x7fffffffu);
     const float ox = na.x, oy = na.y, oz = na.z; // the node's own centre
@@ -747,7 +756,7 @@ __device__ __forceinline__ void walk_group(const DevState &D, const KParams &K, 
   t = t_all;
   tick<Count>(cnt, 15, t, lane);
   if (valid)
-    D.pot[p] = (sum - comp) * K.G_over_a;
+    pot[p] = (sum - comp) * K.G_over_a;
 }
 
 // One 32-target chunk: its subhalo, targets and self terms (as the
@@ -777,9 +786,9 @@ __device__ __forceinline__ void walk_chunk(const DevState &D, const KParams &K, 
   }
   const int root = D.src_off[s] + 2 * D.X[D.src_off[s]];
   if (D.wrap[s])
-    walk_group<true, Count>(D, K, s, root, lane, valid, p, x, self, sh, cnt);
+    walk_group<true, Count, false>(D.nodes, D.pot, K, root, lane, valid, p, x, self, sh, cnt);
   else
-    walk_group<false, Count>(D, K, s, root, lane, valid, p, x, self, sh, cnt);
+    walk_group<false, Count, false>(D.nodes, D.pot, K, root, lane, valid, p, x, self, sh, cnt);
 }
 
 // With walk counters, the chunks (key order) are split into `nranges`

@@ -135,7 +135,8 @@ typedef struct hbtg_stats
   int64_t interactions;       /* node/particle interactions evaluated by the tree walks (if counted) */
   int64_t tree_nodes;         /* internal nodes built, summed over iterations */
   double ms_total;            /* wall time of the device part of the last call (CUDA events) */
-  double ms_walk;             /* summed tree-walk kernel time (CUDA events) */
+  double ms_walk;             /* summed tree-walk kernel time, and that of the kernels which run the last
+                                 iterations of small subhaloes whole, walks included (CUDA events) */
   double ms_plan;             /* per-iteration planning: packing scans and host reads */
   double ms_tree;             /* tree builds: bounding cubes, keys, sorts, cells */
   double ms_part;             /* energies, partition, sort of the removed tails */
