@@ -1395,6 +1395,26 @@ struct KahanF
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
+// Sum of floats with the rounding errors kept (two-sum): hi + lo is exact up
+// to the rounding of lo.
+struct PairSum
+{
+  float hi = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(float v)
+  {
+    const float t = __fadd_rn(hi, v), b = __fsub_rn(t, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
+    hi = t;
+  }
+  __device__ __forceinline__ void add(const PairSum &o)
+  {
+    add(o.hi);
+    lo = __fadd_rn(lo, o.lo);
+  }
+  // an infinite sum has no error term
+  __device__ __forceinline__ double value() const { return isfinite(lo) ? (double)hi + (double)lo : (double)hi; }
+};
+
 // Mass-weighted coordinate of a particle in the centre-of-mass sums, about the
 // bound set's first particle at o.
 __device__ __forceinline__ float com_offset(float x, float o, float m, const KParams &K)

@@ -80,45 +80,64 @@ __global__ void k_prop_init(PropState P)
     P.shape[12 * s + q] = 0.;
 }
 
-// Items: distances, masses, sort keys; shape sums (CalculateShape skips the
-// first bound particle, the centre itself).  Each thread takes
-// kItemsPerThread consecutive items and flushes its double sums per subhalo.
-__global__ void k_prop_items(PropState P, int total)
+// Adds a warp's 12 pair sums over the lanes with `in` to subhalo seg's shape.
+__device__ __forceinline__ void add_shape(const PropState &P, int seg, bool in, PairSum (&acc)[12])
 {
-  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * kItemsPerThread;
-  if (first >= total)
-    return;
-  int s = find_segment<int>(P.fin_off, P.S, (int)first);
-  double acc[12];
+  const int lane = threadIdx.x & 31;
+  double mine = 0.;
+#pragma unroll
   for (int q = 0; q < 12; q++)
-    acc[q] = 0.;
-  auto flush = [&](int seg) {
-    for (int q = 0; q < 12; q++)
-      if (acc[q] != 0.)
-      {
-        atomicAdd(&P.shape[12 * seg + q], acc[q]);
-        acc[q] = 0.;
-      }
-  };
-  const int last = (int)min((long long)total, first + kItemsPerThread);
-  for (int j = (int)first; j < last; j++)
   {
-    if (j >= P.fin_off[s + 1])
-    {
-      flush(s);
-      s = find_segment<int>(P.fin_off, P.S, j);
-    }
+    PairSum t;
+    if (in)
+      t = acc[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      t.add(PairSum{__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o)});
+    if (lane == q)
+      mine = t.value();
+  }
+  if (lane < 12 && mine != 0.)
+    atomicAdd(&P.shape[12 * seg + lane], mine);
+}
+
+// Items: distances, masses, sort keys; shape sums (CalculateShape skips the
+// first bound particle, the centre itself).  A warp takes kPropRows rows of 32
+// consecutive items and keeps the 12 sums in error-free float pairs (FP64 is
+// scarce on this GPU: 24 operations an item held this kernel at 443 us on
+// 3.3e6 items, with 16 strided items a thread) until the subhalo changes;
+// then one double atomic per sum.  Bound by the gathers of positions and
+// masses.
+constexpr int kPropRows = 8;
+__global__ void __launch_bounds__(256) k_prop_items(PropState P, int total)
+{
+  const int lane = threadIdx.x & 31;
+  const long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kPropRows * kWarp);
+  if (first >= total) // whole warps
+    return;
+  PairSum acc[12];
+  int cur = -1; // subhalo that acc belongs to
+#pragma unroll 1
+  for (int r = 0; r < kPropRows; r++)
+  {
+    const long long jj = first + r * kWarp + lane;
+    const bool valid = jj < total;
+    const int j = (int)min(jj, (long long)total - 1);
+    const int s = find_segment_warp(P.fin_off, P.S, j);
+    const int s0 = __shfl_sync(0xffffffffu, s, 0);
+    const bool one = __shfl_sync(0xffffffffu, s, 31) == s0;
     const int k = j - P.fin_off[s];
     const long long g = P.off[s] + P.order[P.off[s] + k];
     const float *x = P.pos + 3 * g, *c = P.mb_pos + 3 * s;
     const float m = P.mass[g];
-    const float r = periodic_distance_f(c, x, P);
-    P.rr[j] = r;
-    P.mm[j] = m;
-    P.k32[j] = __float_as_uint(r); // r >= 0: the bits order as the values
-    P.val[j] = (uint32_t)j;
-    if (k == 0)
-      continue;
+    const float rr = periodic_distance_f(c, x, P);
+    if (valid)
+    {
+      P.rr[j] = rr;
+      P.mm[j] = m;
+      P.k32[j] = __float_as_uint(rr); // r >= 0: the bits order as the values
+      P.val[j] = (uint32_t)j;
+    }
     float dx = __fsub_rn(x[0], c[0]), dy = __fsub_rn(x[1], c[1]), dz = __fsub_rn(x[2], c[2]);
     if (P.periodic)
     {
@@ -127,21 +146,40 @@ __global__ void k_prop_items(PropState P, int total)
       dz = nearest_f(dz, P.half, P.box);
     }
     const float dx2 = __fmul_rn(dx, dx), dy2 = __fmul_rn(dy, dy), dz2 = __fmul_rn(dz, dz);
-    acc[0] += (double)__fmul_rn(dx2, m);
-    acc[1] += (double)__fmul_rn(__fmul_rn(dx, dy), m);
-    acc[2] += (double)__fmul_rn(__fmul_rn(dx, dz), m);
-    acc[3] += (double)__fmul_rn(dy2, m);
-    acc[4] += (double)__fmul_rn(__fmul_rn(dy, dz), m);
-    acc[5] += (double)__fmul_rn(dz2, m);
+    const float xy = __fmul_rn(dx, dy), xz = __fmul_rn(dx, dz), yz = __fmul_rn(dy, dz);
     const float dr2 = __fdiv_rn(__fadd_rn(__fadd_rn(dx2, dy2), dz2), m);
-    acc[6] += (double)__fdiv_rn(dx2, dr2);
-    acc[7] += (double)__fdiv_rn(__fmul_rn(dx, dy), dr2);
-    acc[8] += (double)__fdiv_rn(__fmul_rn(dx, dz), dr2);
-    acc[9] += (double)__fdiv_rn(dy2, dr2);
-    acc[10] += (double)__fdiv_rn(__fmul_rn(dy, dz), dr2);
-    acc[11] += (double)__fdiv_rn(dz2, dr2);
+    const float v[12] = {__fmul_rn(dx2, m),   __fmul_rn(xy, m),    __fmul_rn(xz, m),    __fmul_rn(dy2, m),
+                         __fmul_rn(yz, m),    __fmul_rn(dz2, m),   __fdiv_rn(dx2, dr2), __fdiv_rn(xy, dr2),
+                         __fdiv_rn(xz, dr2),  __fdiv_rn(dy2, dr2), __fdiv_rn(yz, dr2),  __fdiv_rn(dz2, dr2)};
+    const bool counts = valid && k != 0;
+    if (!one || s0 != cur)
+    { // another subhalo: hand in the sums so far
+      if (cur >= 0)
+        add_shape(P, cur, true, acc);
+#pragma unroll
+      for (int q = 0; q < 12; q++)
+        acc[q] = PairSum();
+      cur = one ? s0 : -1;
+    }
+    if (counts)
+#pragma unroll
+      for (int q = 0; q < 12; q++)
+        acc[q].add(v[q]);
+    if (!one)
+    { // each subhalo of the row by itself
+      for (unsigned left = 0xffffffffu; left;)
+      {
+        const int seg = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+        left &= ~__ballot_sync(0xffffffffu, s == seg);
+        add_shape(P, seg, s == seg && counts, acc);
+      }
+#pragma unroll
+      for (int q = 0; q < 12; q++)
+        acc[q] = PairSum();
+    }
   }
-  flush(s);
+  if (cur >= 0)
+    add_shape(P, cur, true, acc);
 }
 
 // Second sort key: the item's subhalo.
@@ -168,28 +206,81 @@ struct PropMassStore
   __device__ void operator()(long long i, const SegD &v) const { out[i] = v.v; }
 };
 
+// Keeps the largest (v, smallest rank) and the outermost overdensity rank of
+// the lanes with `in` in subhalo seg.  v >= 0, so its bits order as its values.
+__device__ __forceinline__ void keep_profile(const PropState &P, int seg, bool in, unsigned v, int q, int so)
+{
+  const unsigned vm = __reduce_max_sync(0xffffffffu, in ? v : 0u);
+  const unsigned qm = __reduce_min_sync(0xffffffffu, in && v == vm ? (unsigned)q : 0xffffffffu);
+  const int sm = __reduce_max_sync(0xffffffffu, in ? so : -1);
+  if ((threadIdx.x & 31) != 0 || qm == 0xffffffffu)
+    return;
+  atomicMax(&P.vkey[seg], ((unsigned long long)vm << 32) | (unsigned long long)(0xffffffffu - qm));
+  if (sm >= 0)
+    atomicMax(&P.so_rank[seg], sm);
+}
+
 // Per sorted item (rank q of subhalo s): the clamped radius, v = M(<r)/r
 // (the largest kept per subhalo, the first on ties) and the overdensity
-// test (the outermost rank that passes it kept per subhalo).
-__global__ void k_prop_profile(PropState P, const uint32_t *__restrict__ sorted, int total)
+// test (the outermost rank that passes it kept per subhalo).  A warp reduces
+// kPropRows rows of 32 items before its atomics: with two of them per item,
+// all of a large subhalo's on the same words, 3.3e6 items took 548 us; this
+// and k_prop_items' rows brought the whole call from 1525 to 781 us.
+__global__ void __launch_bounds__(256) k_prop_profile(PropState P, const uint32_t *__restrict__ sorted, int total)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = find_segment_warp(P.fin_off, P.S, min(i, total - 1));
-  if (i >= total)
+  const int lane = threadIdx.x & 31;
+  const long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kPropRows * kWarp);
+  if (first >= total) // whole warps
     return;
-  const int q = i - P.fin_off[s];
-  const int nb = P.fin_off[s + 1] - P.fin_off[s];
-  if (nb <= 1)
-    return;
-  float r = P.rr[sorted[i]];
-  if (r < P.soft)
-    r = P.soft; // resolution
-  const float m = __double2float_rn(P.mcum[i]);
-  const float v = __fdiv_rn(m, r);
-  atomicMax(&P.vkey[s],
-            ((unsigned long long)__float_as_uint(v) << 32) | (unsigned long long)(0xffffffffu - (unsigned)q));
-  if (m > __fmul_rn(__fmul_rn(__fmul_rn(P.rho_vir, r), r), r))
-    atomicMax(&P.so_rank[s], q);
+  int cur = -1, best_q = 0, best_so = -1;
+  unsigned best_v = 0u;
+  bool any = false; // this lane's best of subhalo cur
+#pragma unroll 2
+  for (int r = 0; r < kPropRows; r++)
+  {
+    const long long ii = first + r * kWarp + lane;
+    const int i = (int)min(ii, (long long)total - 1);
+    const int s = find_segment_warp(P.fin_off, P.S, i);
+    const int s0 = __shfl_sync(0xffffffffu, s, 0);
+    const bool one = __shfl_sync(0xffffffffu, s, 31) == s0;
+    const int q = i - P.fin_off[s];
+    const bool counts = ii < total && P.fin_off[s + 1] - P.fin_off[s] > 1;
+    float rad = P.rr[sorted[i]];
+    if (rad < P.soft)
+      rad = P.soft; // resolution
+    const float m = __double2float_rn(P.mcum[i]);
+    const unsigned v = __float_as_uint(__fdiv_rn(m, rad));
+    const int so = m > __fmul_rn(__fmul_rn(__fmul_rn(P.rho_vir, rad), rad), rad) ? q : -1;
+    if (!one || s0 != cur)
+    {
+      if (cur >= 0)
+        keep_profile(P, cur, any, best_v, best_q, best_so);
+      cur = one ? s0 : -1;
+      any = false;
+      best_so = -1;
+    }
+    if (!one)
+    {
+      for (unsigned left = 0xffffffffu; left;)
+      {
+        const int seg = __shfl_sync(0xffffffffu, s, __ffs(left) - 1);
+        left &= ~__ballot_sync(0xffffffffu, s == seg);
+        keep_profile(P, seg, s == seg && counts, v, q, so);
+      }
+    }
+    else if (counts)
+    {
+      if (!any || v > best_v)
+      { // ranks ascend: an equal v keeps the first
+        best_v = v;
+        best_q = q;
+      }
+      best_so = max(best_so, so);
+      any = true;
+    }
+  }
+  if (cur >= 0)
+    keep_profile(P, cur, any, best_v, best_q, best_so);
 }
 
 struct PropOut

@@ -102,20 +102,6 @@ __global__ void k_settle_pick(DevState D, KParams K, SettleArgs A)
   A.list[(size_t)c * D.S + atomicAdd(&A.count[c], 1)] = s;
 }
 
-// Sum of floats with the rounding errors kept (two-sum): hi + lo is exact up
-// to the rounding of lo.
-struct PairSum
-{
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(float v)
-  {
-    const float t = __fadd_rn(hi, v), b = __fsub_rn(t, hi);
-    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
-    hi = t;
-  }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
-};
-
 template <int C>
 __device__ __forceinline__ void team_sync()
 {

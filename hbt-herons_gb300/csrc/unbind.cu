@@ -1105,7 +1105,8 @@ int props_run(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, int sna
   const uint32_t *sorted = Q.val;
   if (T > 0)
   {
-    k_prop_items<<<blocks_for(((long long)T + kItemsPerThread - 1) / kItemsPerThread, 256), 256, 0, st>>>(Q, T);
+    const unsigned pb = blocks_for(((long long)T + kPropRows - 1) / kPropRows, 256);
+    k_prop_items<<<pb, 256, 0, st>>>(Q, T);
     launches++;
     HBTG_CUDA(cudaGetLastError());
     // by distance, then stably by subhalo
@@ -1129,7 +1130,7 @@ int props_run(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, int sna
     sorted = v;
     SegD *sscr = P.get<SegD>(S_PR_SCR, scan_scratch_elems<SegD>(T));
     scan_load_store<SegD, true>(PropMassLoad{Q, sorted}, PropMassStore{Q.mcum}, T, sscr, st, &launches);
-    k_prop_profile<<<blocks_for(T, 256), 256, 0, st>>>(Q, sorted, T);
+    k_prop_profile<<<pb, 256, 0, st>>>(Q, sorted, T);
     launches++;
     HBTG_CUDA(cudaGetLastError());
   }
