@@ -225,19 +225,26 @@ struct IterationDriver
     tree_nodes += internal;
     k_tree_emit<<<grid_for(src_total, 128), 128, 0, st>>>(D, K, src_total);
     launches++;
-    // cell multipoles (or bounding boxes) bottom-up, one launch per non-empty
-    // level, deepest first
-    for (int L = 21; L >= 0; L--) // keys have 21 digits: no cell below level 21
+    // cell multipoles (or bounding boxes) bottom-up, deepest level first: one
+    // launch per level of many cells, one per run of levels of few
+    LevelOffsets lv{};
+    for (int l = 0; l + 1 < kLevels; l++)
+      lv.off[l + 1] = lv.off[l] + per_level[l];
+    for (int L = 21; L >= 0;) // keys have 21 digits: no cell below level 21
     {
       if (per_level[L] <= 0)
+      {
+        L--;
         continue;
-      const unsigned mg =
-        std::max(1u, std::min(grid_for(per_level[L], 256), (unsigned)sm_count * (unsigned)moments_blocks_per_sm));
+      }
+      int last = L; // the run L, L - 1, ..., last
+      while (per_level[L] <= kMomentsFew && last > 0 && per_level[last - 1] <= kMomentsFew)
+        last--;
       if (geometric)
-        k_tree_bounds<<<mg, 256, 0, st>>>(D, L);
+        launch_moments<true>(lv, L, last);
       else
-        k_tree_moments<<<mg, 256, 0, st>>>(D, L);
-      launches++;
+        launch_moments<false>(lv, L, last);
+      L = last - 1;
     }
     if (geometric)
     {
@@ -245,6 +252,30 @@ struct IterationDriver
       launches++;
     }
     check();
+  }
+
+  template <bool Geometric>
+  void launch_moments(const LevelOffsets &lv, int L0, int L1)
+  {
+    launches++;
+    if (L0 == L1)
+    {
+      const unsigned mg = std::max(1u, std::min(grid_for(lv.off[L0 + 1] - lv.off[L0], 256),
+                                                (unsigned)sm_count * (unsigned)moments_blocks_per_sm));
+      k_tree_moments<Geometric, false><<<mg, 256, 0, st>>>(D.nodes, D.cell_list, lv, L0, L1);
+      return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kMomentsCluster);
+    cfg.blockDim = dim3(kMomentsThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kMomentsCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    mem.check(cudaLaunchKernelEx(&cfg, k_tree_moments<Geometric, true>, D.nodes, (const int *)D.cell_list, lv, L0, L1));
   }
 
   // Targets of the correction walks in key order (see k_tgt_flags); `total`
