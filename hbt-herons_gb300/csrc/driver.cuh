@@ -12,6 +12,7 @@
 //   int *scan_scratch(long long n)               scratch for scan<int>(n)
 //   int *radix_table(long long n)                table for radix_sort_pairs(n)
 //   int *radix_scan_scratch(long long n)
+//   unsigned *ticket()                           a zero for the scans and sorts (null: without it)
 //   int *cell_list(long long cells)              per-level cell lists of one tree (may throw)
 //   int *level_counts()                          2 kLevels ints
 //   float4 *tree_slots(long long slots)          tree storage (may throw when too large)
@@ -117,7 +118,7 @@ struct IterationDriver
   {
     // an int scratch for 8 (n + 1) items covers scan_scratch_elems<I4c>(n + 1) I4cs
     I4c *scr = reinterpret_cast<I4c *>(mem.scan_scratch(8 * (n + 1)));
-    scan_load_store<I4c, false>(Count4Load{c0, c1, c2, c3}, Count4Store{o0, o1, o2, o3}, n + 1, scr, st, &launches);
+    scan_load_store<I4c, false>(Count4Load{c0, c1, c2, c3}, Count4Store{o0, o1, o2, o3}, n + 1, scr, st, &launches, mem.ticket());
     check();
     int *outs[4] = {o0, o1, o2, o3};
     for (int k = 0; k < 4; k++)
@@ -133,7 +134,7 @@ struct IterationDriver
   // Exclusive scan of n counts plus a trailing zero; returns the total.
   int scan_counts(const int *cnt, int *offs, long long n)
   {
-    scan<int, false>(cnt, offs, n + 1, mem.scan_scratch(n + 1), st, &launches);
+    scan<int, false>(cnt, offs, n + 1, mem.scan_scratch(n + 1), st, &launches, mem.ticket());
     check();
     return read_int(offs + n);
   }
@@ -145,7 +146,7 @@ struct IterationDriver
     int *table = mem.radix_table(total), *scr = mem.radix_scan_scratch(total);
     const bool flip =
       radix_sort_pairs<uint32_t>(D.k32, D.val, D.k32_alt, D.val_alt, total, 0, 32, table, scr, st, &launches,
-                                 block_sort_max);
+                                 mem.ticket(), block_sort_max);
     uint32_t *v = flip ? D.val_alt : D.val;
     uint32_t *v_other = flip ? D.val : D.val_alt;
     if (S > 1 && seg_bits > 0)
@@ -154,7 +155,7 @@ struct IterationDriver
       launches++;
       const bool f2 =
         radix_sort_pairs<uint32_t>(D.k32, v, D.k32_alt, v_other, total, 0, seg_bits, table, scr, st, &launches,
-                                   block_sort_max);
+                                   mem.ticket(), block_sort_max);
       v = f2 ? v_other : v;
     }
     check();
@@ -168,7 +169,7 @@ struct IterationDriver
     int *table = mem.radix_table(total), *scr = mem.radix_scan_scratch(total);
     const bool flip =
       radix_sort_pairs<unsigned long long>(D.key, D.val, D.key_alt, D.val_alt, total, 0, 63, table, scr, st,
-                                           &launches, block_sort_max);
+                                           &launches, mem.ticket(), block_sort_max);
     if (flip)
     {
       std::swap(D.key, D.key_alt);
@@ -179,7 +180,7 @@ struct IterationDriver
       k_segkeys_iota<<<grid_for(total, 256), 256, 0, st>>>(D.val, D.seg_of, D.k32, D.perm, total);
       launches++;
       const bool f2 = radix_sort_pairs<uint32_t>(D.k32, D.perm, D.k32_alt, D.perm_alt, total, 0, seg_bits, table,
-                                                 scr, st, &launches, block_sort_max);
+                                                 scr, st, &launches, mem.ticket(), block_sort_max);
       const uint32_t *perm = f2 ? D.perm_alt : D.perm;
       k_gather_keys<<<grid_for(total, 256), 256, 0, st>>>(D.key, D.val, perm, D.key_alt, D.val_alt, total);
       launches++;
@@ -210,7 +211,7 @@ struct IterationDriver
     launches++;
     check();
     // the cell total and the cells per level (k_tree_count's histogram) in one host read
-    scan<int, false>(D.cnt, D.X, src_total + 1, mem.scan_scratch(src_total + 1), st, &launches);
+    scan<int, false>(D.cnt, D.X, src_total + 1, mem.scan_scratch(src_total + 1), st, &launches, mem.ticket());
     check();
     int counts[1 + kLevels];
     mem.check(cudaMemcpyAsync(&counts[0], D.X + src_total, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -286,7 +287,7 @@ struct IterationDriver
       return;
     k_tgt_flags<<<grid_for(total + 1, 256), 256, 0, st>>>(D, total);
     launches++;
-    scan<int, false>(D.flags, D.F, total + 1, mem.scan_scratch(total + 1), st, &launches);
+    scan<int, false>(D.flags, D.F, total + 1, mem.scan_scratch(total + 1), st, &launches, mem.ticket());
     k_tgt_scatter<<<grid_for(total, 256), 256, 0, st>>>(D, total);
     launches++;
     check();
@@ -434,7 +435,7 @@ struct IterationDriver
         k_part_flags<<<grid_for(part_total + 1, 256), 256, 0, st>>>(D, part_total);
         launches += 2;
         check();
-        scan<int, false>(D.flags, D.F, part_total + 1, mem.scan_scratch(part_total + 1), st, &launches);
+        scan<int, false>(D.flags, D.F, part_total + 1, mem.scan_scratch(part_total + 1), st, &launches, mem.ticket());
         k_part_count<<<sb, 256, 0, st>>>(D);
         k_part_scatter<<<grid_for(part_total, 256), 256, 0, st>>>(D, part_total);
         k_part_copy<<<grid_for(part_total, 256), 256, 0, st>>>(D, part_total);

@@ -163,6 +163,7 @@ struct StaticMem
     return table;
   }
   int *radix_scan_scratch(long long n) { return scan_scratch(radix_table_elems(std::max<long long>(n, 1)) + 1); }
+  unsigned *ticket() { return nullptr; }
   int *cell_list(long long n)
   {
     if (n > (long long)kCells)

@@ -229,6 +229,7 @@ struct hbtg_handle
   cudaEvent_t copy_events[7] = {};          // host-pointer calls: copy phases and the side streams
   cudaEvent_t epilogue_wait = nullptr;      // set for one call: the epilogue waits for this event
   Pool pool;
+  unsigned *ticket = nullptr;               // a device zero for the last-block scans (primitives.cuh)
   hbtg_stats stats{};
   bool count_interactions = false;
   std::vector<cudaEvent_t> walk_events;
@@ -350,6 +351,7 @@ struct PoolMem
                                          std::max<long long>(radix_table_elems(std::max<long long>(n, 1)) + 1,
                                                              256LL * 4096)));
   }
+  unsigned *ticket() { return H->ticket; }
   int *cell_list(long long cells) { return H->pool.get<int>(S_CELLS, (size_t)std::max<long long>(cells, 1)); }
   int *level_counts() { return H->pool.get<int>(S_LVL, 2 * kLevels); }
   float4 *tree_slots(long long slots)
@@ -924,7 +926,8 @@ int pot_call(void *arg)
     bits++;
   // the values carried along are not read: the key alone names the target
   const bool flip = radix_sort_pairs<uint32_t>(D.k32, D.val_alt, D.k32_alt, D.perm_alt, c.nt, 0, bits,
-                                               mem.radix_table(c.nt), mem.radix_scan_scratch(c.nt), st, &R.launches);
+                                               mem.radix_table(c.nt), mem.radix_scan_scratch(c.nt), st, &R.launches,
+                                               H->ticket);
   k_pot_order<<<blocks_for(c.nt, 256), 256, 0, st>>>(D, flip ? D.k32_alt : D.k32, (int)c.nt);
   k_pot_plan<<<1, 32, 0, st>>>(D, (int)c.nt, 1);
   R.check();
@@ -1092,7 +1095,7 @@ int props_run(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, int sna
   k_prop_init<<<blocks_for(S + 1, 256), 256, 0, st>>>(Q);
   launches++;
   HBTG_CUDA(cudaGetLastError());
-  scan<int, false>(Q.cnt, Q.fin_off, S + 1, P.get<int>(S_SCRATCH, scan_scratch_elems<int>(S + 1)), st, &launches);
+  scan<int, false>(Q.cnt, Q.fin_off, S + 1, P.get<int>(S_SCRATCH, scan_scratch_elems<int>(S + 1)), st, &launches, H->ticket);
   const int T = read_int(Q.fin_off + S, st);
   const size_t t1 = (size_t)std::max(T, 1);
   Q.rr = P.get<float>(S_PR_RR, t1);
@@ -1114,7 +1117,7 @@ int props_run(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, int sna
     int *scr = P.get<int>(S_SCRATCH, scan_scratch_elems<int>(std::max<long long>(radix_table_elems(T) + 1,
                                                                                       256LL * 4096)));
     const bool f1 = radix_sort_pairs<uint32_t>(Q.k32, Q.val, Q.k32_alt, Q.val_alt, T, 0, 32, table, scr, st,
-                                               &launches);
+                                               &launches, H->ticket);
     uint32_t *v = f1 ? Q.val_alt : Q.val, *v_other = f1 ? Q.val : Q.val_alt;
     int bits = 0;
     while ((1LL << bits) < S)
@@ -1124,12 +1127,12 @@ int props_run(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, int sna
       k_prop_segkeys<<<blocks_for(T, 256), 256, 0, st>>>(Q, v, Q.k32, T);
       launches++;
       const bool f2 = radix_sort_pairs<uint32_t>(Q.k32, v, Q.k32_alt, v_other, T, 0, bits, table, scr, st,
-                                                 &launches);
+                                                 &launches, H->ticket);
       v = f2 ? v_other : v;
     }
     sorted = v;
     SegD *sscr = P.get<SegD>(S_PR_SCR, scan_scratch_elems<SegD>(T));
-    scan_load_store<SegD, true>(PropMassLoad{Q, sorted}, PropMassStore{Q.mcum}, T, sscr, st, &launches);
+    scan_load_store<SegD, true>(PropMassLoad{Q, sorted}, PropMassStore{Q.mcum}, T, sscr, st, &launches, H->ticket);
     k_prop_profile<<<pb, 256, 0, st>>>(Q, sorted, T);
     launches++;
     HBTG_CUDA(cudaGetLastError());
@@ -1289,7 +1292,7 @@ int reassign_run(hbtg_handle *H, const hbtg_params *p, const hbtg_reassign *r, i
   k_re_flags<<<blocks_for(N + 1, 256), 256, 0, st>>>(Q, N);
   launches++;
   HBTG_CUDA(cudaGetLastError());
-  scan<int, false>(Q.flags, Q.rank, N + 1, P.get<int>(S_SCRATCH, scan_scratch_elems<int>(N + 1)), st, &launches);
+  scan<int, false>(Q.flags, Q.rank, N + 1, P.get<int>(S_SCRATCH, scan_scratch_elems<int>(N + 1)), st, &launches, H->ticket);
   const int T = read_int(Q.rank + N, st);
   const size_t t1 = (size_t)std::max(T, 1);
   Q.tg = P.get<int>(S_RE_TG, t1);
@@ -1366,7 +1369,8 @@ int reassign_run(hbtg_handle *H, const hbtg_params *p, const hbtg_reassign *r, i
     k_re_queries<<<blocks_for(N, 256), 256, 0, st>>>(Q, D, N);
     launches++;
     if (radix_sort_pairs<unsigned long long>(qkey, qval, qkey_alt, qval_alt, nq, 0, 3 * kReDigits + bits,
-                                             mem.radix_table(nq), mem.radix_scan_scratch(nq), st, &launches))
+                                             mem.radix_table(nq), mem.radix_scan_scratch(nq), st, &launches,
+                                             H->ticket))
     {
       Q.qkey = qkey_alt;
       Q.qval = qval_alt;
@@ -1513,6 +1517,14 @@ int hbtg_create(hbtg_handle **handle, int device)
     delete h;
     return HBTG_ERR_CUDA;
   }
+  if (cudaMalloc(&h->ticket, 256) != cudaSuccess || cudaMemset(h->ticket, 0, 256) != cudaSuccess)
+  {
+    cudaGetLastError();
+    cudaFree(h->ticket);
+    cudaStreamDestroy(h->stream);
+    delete h;
+    return HBTG_ERR_NOMEM;
+  }
   h->walk_events.resize(2);
   for (auto &e : h->walk_events)
     if (cudaEventCreate(&e) != cudaSuccess)
@@ -1542,6 +1554,7 @@ int hbtg_destroy(hbtg_handle *h)
     return HBTG_ERR_INVALID;
   cudaSetDevice(h->device);
   h->pool.release();
+  cudaFree(h->ticket);
   for (auto &e : h->walk_events)
     cudaEventDestroy(e);
   for (auto &e : h->phase_events)

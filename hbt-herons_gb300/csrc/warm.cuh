@@ -780,7 +780,7 @@ long long first_test(IterationDriver<Mem> &R, const WarmBufs &W)
     R.build_tree(src_total);
     k_first_tgt_flags<<<grid_for(src_total + 1, 256), 256, 0, st>>>(D, W, src_total);
     R.launches++;
-    scan<int, false>(D.flags, D.F, src_total + 1, R.mem.scan_scratch(src_total + 1), st, &R.launches);
+    scan<int, false>(D.flags, D.F, src_total + 1, R.mem.scan_scratch(src_total + 1), st, &R.launches, R.mem.ticket());
     k_first_tgt_scatter<<<grid_for(src_total, 256), 256, 0, st>>>(D, src_total);
     R.launches++;
     R.check();
@@ -794,7 +794,7 @@ long long first_test(IterationDriver<Mem> &R, const WarmBufs &W)
     k_readmit_energy<<<grid_for(part_total + 1, 256), 256, 0, st>>>(D, R.K, part_total);
     k_first_flags<<<grid_for(tail_total + 1, 256), 256, 0, st>>>(D, tail_total);
     R.launches += 2;
-    scan<int, false>(D.flags, D.F, tail_total + 1, R.mem.scan_scratch(tail_total + 1), st, &R.launches);
+    scan<int, false>(D.flags, D.F, tail_total + 1, R.mem.scan_scratch(tail_total + 1), st, &R.launches, R.mem.ticket());
     R.check();
     kept = R.read_int(D.F + tail_total);
     k_readmit_scatter<<<grid_for(tail_total, 256), 256, 0, st>>>(D, tail_total);
@@ -824,8 +824,8 @@ void warm_run(IterationDriver<Mem> &R, const WarmBufs &W, WarmCounters &C, bool 
   {
     k_warm_flags<<<grid_for(D.N + 1, 256), 256, 0, st>>>(D, W);
     R.launches++;
-    scan<int, false>(D.flags, D.F, D.N + 1, R.mem.scan_scratch(D.N + 1), st, &R.launches);
-    scan<int, false>(D.cnt, D.X, D.N + 1, R.mem.scan_scratch(D.N + 1), st, &R.launches);
+    scan<int, false>(D.flags, D.F, D.N + 1, R.mem.scan_scratch(D.N + 1), st, &R.launches, R.mem.ticket());
+    scan<int, false>(D.cnt, D.X, D.N + 1, R.mem.scan_scratch(D.N + 1), st, &R.launches, R.mem.ticket());
     R.check();
   }
   else
