@@ -414,8 +414,10 @@ struct IterationDriver
       global_iter++;
       if (K.max_sample > 0)
       { // upscale factors of the subsampled subhaloes
-        k_upscale<<<(unsigned)std::min(S, 65535), 256, 0, st>>>(D, K);
-        launches++;
+        if (part_total > 0)
+          k_upscale_sums<<<grid_for((part_total + kUpscaleRows - 1) / kUpscaleRows, 256), 256, 0, st>>>(D, K, part_total);
+        k_upscale<<<sb, 256, 0, st>>>(D, K);
+        launches += 2;
         check();
       }
       if (src_total > 0)
