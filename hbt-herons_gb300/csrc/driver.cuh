@@ -190,8 +190,7 @@ struct IterationDriver
     check();
   }
 
-  // geometric: per-cell bounding boxes and leaf source indices (k_tree_bounds,
-  // k_tree_leaf_ids) instead of mass moments.
+  // geometric: per-cell bounding boxes (cell_bounds) instead of mass moments.
   void build_tree(int src_total, bool geometric = false)
   {
     if (src_total <= 0)
@@ -246,11 +245,6 @@ struct IterationDriver
       else
         launch_moments<false>(lv, L, last);
       L = last - 1;
-    }
-    if (geometric)
-    {
-      k_tree_leaf_ids<<<grid_for(src_total, 256), 256, 0, st>>>(D, src_total);
-      launches++;
     }
     check();
   }

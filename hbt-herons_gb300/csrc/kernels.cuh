@@ -1221,8 +1221,8 @@ __device__ __forceinline__ void cell_moments(float4 *nodes, int slot)
 
 // Geometric trees (neighbour searches): a cell's bounding box of its
 // particles instead of its mass moments, from its children.  Slots of a cell:
-// (lo.x, lo.y, lo.z, -threshold), (hi.x, skip, hi.y, hi.z); a leaf's w holds
-// its source index (int bits) once k_tree_leaf_ids has run.
+// (lo.x, lo.y, lo.z, -threshold), (hi.x, skip, hi.y, hi.z); a leaf's w is
+// free for the search's own use (a number whose sign bit is clear).
 __device__ __forceinline__ void cell_bounds(float4 *nodes, int slot)
 {
   const int end = __float_as_int(nodes[slot + 1].y);
@@ -1284,16 +1284,6 @@ __global__ void __launch_bounds__(kMomentsThreads)
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
   }
-}
-
-// Leaf slots of a geometric tree carry their source index in w.
-__global__ void k_tree_leaf_ids(DevState D, int total)
-{
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= total)
-    return;
-  const int slot = j + 2 * D.X[j] + 2 * D.cnt[j];
-  reinterpret_cast<int *>(&D.nodes[slot])[3] = (int)D.val[j];
 }
 
 // ---------------------------------------------------------------------------

@@ -49,6 +49,7 @@ struct ReState
   int *flags, *rank;         // [N+1] tracer flags and their exclusive scan
   int *tg;                   // [T] particle of each packed tracer
   int *tsub;                 // [T] subhalo of each packed tracer
+  float4 *raw;               // [T] tracers in the trees' leaf order: raw position, packed tracer (int bits)
   unsigned long long *qkey;  // [N - T] search order: group, then the top digits of the particle's tree key
   uint32_t *qval;            // [N - T] the non-tracers, in search order once sorted by qkey
   int tracer_mask;
@@ -181,10 +182,13 @@ struct ReRadii
 // The first search j < 4096 that collects a tracer at (d2, dmax): the radii
 // do not decrease, so a binary search over the table finds it; past the
 // table's end (an initial radius so small that it does not reach infinity
-// there) the searches go on one by one.
+// there) the searches go on one by one.  dmax <= R and d2 < R * R (a float)
+// are decided on the floats next to dmax (above) and d2 (below), which compare
+// with a float as they do.
 __device__ __forceinline__ int re_jmin(double d2, double dmax, const float *radii, int n)
 {
-  auto takes = [&](float R) { return dmax <= (double)R && d2 < (double)__fmul_rn(R, R); };
+  const float up = __double2float_ru(dmax), down = __double2float_rd(d2);
+  auto takes = [&](float R) { return up <= R && down < __fmul_rn(R, R); };
   int lo = 0, hi = n;
   while (lo < hi)
   {
@@ -240,15 +244,86 @@ __global__ void k_re_queries(ReState R, DevState D, long long n)
   R.qval[i] = (uint32_t)g;
 }
 
+// Leaf order of the tracers: the leaf's w holds its place j among them, raw[j]
+// the raw position and the packed tracer.
+__global__ void k_re_leaves(ReState R, DevState D, int total)
+{
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= total)
+    return;
+  const int t = (int)D.val[j];
+  const float *x = R.pos + 3 * (long long)R.tg[t];
+  R.raw[j] = make_float4(x[0], x[1], x[2], __int_as_float(t));
+  reinterpret_cast<int *>(&D.nodes[j + 2 * D.X[j] + 2 * D.cnt[j]])[3] = j;
+}
+
+// Squared distance in FP32 from the raw positions: within kReLoose (relative)
+// of the exact one.
+constexpr float kReLoose = 2e-6f;
+__device__ __forceinline__ float re_r2(const float4 &a, const float *q, const ReState &R)
+{
+  float d[3] = {__fsub_rn(a.x, q[0]), __fsub_rn(a.y, q[1]), __fsub_rn(a.z, q[2])};
+  if (R.periodic)
+  { // without rounding the large intermediate: one operand of a wrapped difference is beyond half the box
+    const float p[3] = {a.x, a.y, a.z};
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      d[k] = d[k] > R.half    ? __fsub_rn(__fsub_rn(p[k], R.box), q[k])
+             : d[k] < -R.half ? __fsub_rn(p[k], __fsub_rn(q[k], R.box))
+                              : d[k];
+  }
+  return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+}
+
+// Squared reach of a search whose k-th squared distance is at most r2: a cell
+// or leaf beyond it, by its unwrapped floats, is passed over (eps covers their
+// rounding, the factor that of the arithmetic).
+__device__ __forceinline__ float re_reach2(float r2, const ReState &R)
+{
+  const float r = __fsqrt_ru(r2) + R.eps;
+  return r * r * (1.f + 4e-6f);
+}
+
+// Visits the leaves of group h's tree within reach of uq, in tree order, up to
+// the root's end; take(j, reach) may shrink the reach.
+template <typename Take>
+__device__ __forceinline__ void re_walk(const float4 *T, int root, const float *uq, float reach, Take take)
+{
+  const int end = __float_as_int(T[root + 1].y);
+  int idx = root;
+  while (idx < end)
+  {
+    const float4 a = T[idx], b = T[idx + 1]; // both at once: one latency a node (a padding slot follows the tree)
+    if (slot_is_cell(a.w))
+    {
+      const float gx = fmaxf(fmaxf(a.x - uq[0], uq[0] - b.x), 0.f);
+      const float gy = fmaxf(fmaxf(a.y - uq[1], uq[1] - b.z), 0.f);
+      const float gz = fmaxf(fmaxf(a.z - uq[2], uq[2] - b.w), 0.f);
+      idx = gx * gx + gy * gy + gz * gz > reach ? max(__float_as_int(b.y), idx + 2) : idx + 2;
+      continue;
+    }
+    idx++;
+    const float fx = a.x - uq[0], fy = a.y - uq[1], fz = a.z - uq[2];
+    if (!(fx * fx + fy * fy + fz * fz > reach))
+      take(__float_as_int(a.w), reach);
+  }
+}
+
 // One thread per non-tracer, in search order: dest = the subhalo it moves to
-// (dest holds -1 before).  Bound by the latency of the tree's slots and of
-// the candidates' positions; before, each thread walked from the root with
-// no bound until it held k tracers, in the particles' list order: a call
-// over 3e5 particles in 40 groups (k = 10) took 45.2 ms, now 3.34 ms.
+// (dest holds -1 before).  The k nearest are searched in FP32 (FP64, with its
+// 16 cycles an SM and instruction, held a first version): a first bound from
+// 2k neighbours in key order, then the k + 2 smallest FP32 distances; the
+// exact distances of these decide, unless more tracers than that lie within
+// the FP32 error of the k-th (coincident ones), when the search is repeated
+// with exact distances.  Bound by the latency of the tree's slots.  From the
+// tree's root without a bound, in the particles' list order, a call over 3e5
+// particles in 40 groups (k = 10) took 45.2 ms; with exact distances
+// throughout 3.26 ms, now 1.55 ms.
 template <int kMax>
 __global__ void __launch_bounds__(128)
   k_re_query(ReState R, DevState D, const __grid_constant__ ReRadii table, long long nq)
 {
+  constexpr int kKeep = kMax + 2;
   __shared__ float radii[kReRadii];
   const int n_radii = table.n;
   for (int j = threadIdx.x; j < n_radii; j += blockDim.x)
@@ -263,32 +338,30 @@ __global__ void __launch_bounds__(128)
   if (nt == 0 || D.src_cnt[h] == 0)
     return;
   const int k = R.k;
-  const float *q = R.pos + 3 * g;
+  const float q[3] = {R.pos[3 * g], R.pos[3 * g + 1], R.pos[3 * g + 2]};
   const float *ref = R.pos + 3 * (long long)R.tg[D.off[h]];
   const float uq[3] = {unwrap(q[0], ref[0], R), unwrap(q[1], ref[1], R), unwrap(q[2], ref[2], R)};
-  // the k nearest so far, ascending; equal distances keep the earlier in the tree
-  double bd[kMax];
-  int bi[kMax];
+  const int seg0 = D.src_off[h], seg1 = seg0 + nt;
+  const int root = seg0 + 2 * D.X[seg0];
+  float fd[kKeep]; // FP32 squared distances, ascending
+  int fj[kKeep];   // their places in leaf order
   int cnt = 0;
-  auto insert = [&](double d2, int t) {
-    int at = cnt < k ? cnt : k - 1;
-    while (at > 0 && bd[at - 1] > d2)
+  auto keep = [&](float r2, int j, int cap) {
+    int at = cnt < cap ? cnt : cap - 1;
+    while (at > 0 && fd[at - 1] > r2)
     {
-      bd[at] = bd[at - 1];
-      bi[at] = bi[at - 1];
+      fd[at] = fd[at - 1];
+      fj[at] = fj[at - 1];
       at--;
     }
-    bd[at] = d2;
-    bi[at] = t;
-    cnt += cnt < k;
+    fd[at] = r2;
+    fj[at] = j;
+    cnt += cnt < cap;
   };
-  // first bound: the k-th distance among 2k neighbours in key order.  All of
-  // the k nearest lie within it, so the search below takes the same ones, in
-  // the same order, as without it.
-  double bound = INFINITY;
+  // the k-th distance among 2k neighbours in key order bounds the k-th of all
+  float bound = INFINITY;
   if (nt >= k)
   {
-    const int seg0 = D.src_off[h], seg1 = seg0 + nt;
     const unsigned long long key = re_place(uq, D.keyp + 12 * h);
     int lo = seg0, hi = seg1;
     while (lo < hi)
@@ -302,64 +375,84 @@ __global__ void __launch_bounds__(128)
     const int j0 = max(seg0, min(lo - k, seg1 - 2 * k)), j1 = min(seg1, j0 + 2 * k);
     for (int j = j0; j < j1; j++)
     {
-      double dmax;
-      const double d2 = re_d2(R.pos + 3 * (long long)R.tg[D.val[j]], q, R, dmax);
-      if (cnt < k || d2 < bd[cnt - 1])
-        insert(d2, 0);
+      const float r2 = re_r2(R.raw[j], q, R);
+      if (cnt < k || r2 < fd[cnt - 1])
+        keep(r2, j, k);
     }
-    if (bd[k - 1] < bound) // not for a NaN
-      bound = bd[k - 1];
+    if (fd[k - 1] < bound) // not for a NaN
+      bound = fd[k - 1] * (1.f + 2.f * kReLoose);
     cnt = 0;
   }
-  // A cell or leaf farther than the bound, with a margin for the unwrapped
-  // floats (eps) and for the FP32 arithmetic of the distance, is passed over.
-  auto reach2 = [&](double b) {
-    const float r = __double2float_ru(sqrt(b)) + R.eps;
-    return r * r * (1.f + 4e-6f);
-  };
-  float reach = reach2(bound);
-  const float4 *T = D.nodes;
-  const int root = D.src_off[h] + 2 * D.X[D.src_off[h]];
-  const int end = __float_as_int(T[root + 1].y);
-  int idx = root;
-  while (idx < end)
-  {
-    const float4 a = T[idx];
-    if (slot_is_cell(a.w))
+  const int cap = k + 2;
+  re_walk(D.nodes, root, uq, re_reach2(bound, R), [&](int j, float &reach) {
+    const float r2 = re_r2(R.raw[j], q, R);
+    if (cnt < cap ? !(r2 > bound) : r2 < fd[cap - 1])
     {
-      const float4 b = T[idx + 1];
-      const float gx = fmaxf(fmaxf(a.x - uq[0], uq[0] - b.x), 0.f);
-      const float gy = fmaxf(fmaxf(a.y - uq[1], uq[1] - b.z), 0.f);
-      const float gz = fmaxf(fmaxf(a.z - uq[2], uq[2] - b.w), 0.f);
-      idx = gx * gx + gy * gy + gz * gz > reach ? max(__float_as_int(b.y), idx + 2) : idx + 2;
-      continue;
-    }
-    idx++;
-    const float fx = a.x - uq[0], fy = a.y - uq[1], fz = a.z - uq[2];
-    if (fx * fx + fy * fy + fz * fz > reach)
-      continue;
-    const int t = __float_as_int(a.w); // the packed tracer (k_tree_leaf_ids)
-    double dmax;
-    const double d2 = re_d2(R.pos + 3 * (long long)R.tg[t], q, R, dmax);
-    if (cnt < k ? !(d2 > bound) : d2 < bd[k - 1])
-    {
-      insert(d2, t);
-      if (cnt == k && bd[k - 1] < bound)
-      {
-        bound = bd[k - 1];
-        reach = reach2(bound);
+      keep(r2, j, cap);
+      if (cnt >= k && fd[k - 1] < bound)
+      { // what lies within the error of the k-th stays in reach
+        bound = fminf(bound, fd[k - 1] * (1.f + 2.f * kReLoose));
+        reach = re_reach2(bound, R);
       }
     }
-  }
+  });
+  // their exact distances, ascending; equal ones in tree order
+  double bd[kKeep], bm[kKeep];
+  int bi[kKeep];
+  auto exact_of = [&](int j, double &dmax) {
+    const float4 a = R.raw[j];
+    const float x[3] = {a.x, a.y, a.z};
+    return re_d2(x, q, R, dmax);
+  };
+  int m = 0;
+  // all that may belong to the k nearest are here unless the list is full of them
+  const bool crowded = cnt == cap && !(fd[cap - 1] > fd[k - 1] * (1.f + 2.f * kReLoose));
+  if (!crowded)
+    for (int e = 0; e < cnt; e++)
+    {
+      double dmax;
+      const double d2 = exact_of(fj[e], dmax);
+      int at = m++;
+      while (at > 0 && (bd[at - 1] > d2 || (bd[at - 1] == d2 && bi[at - 1] > fj[e])))
+      {
+        bd[at] = bd[at - 1];
+        bm[at] = bm[at - 1];
+        bi[at] = bi[at - 1];
+        at--;
+      }
+      bd[at] = d2;
+      bm[at] = dmax;
+      bi[at] = fj[e];
+    }
+  else
+    re_walk(D.nodes, root, uq, re_reach2(bound, R), [&](int j, float &) {
+      double dmax;
+      const double d2 = exact_of(j, dmax);
+      if (m < k || d2 < bd[m - 1])
+      { // the leaves come in tree order: equal distances keep the earlier
+        int at = m < k ? m : k - 1;
+        while (at > 0 && bd[at - 1] > d2)
+        {
+          bd[at] = bd[at - 1];
+          bm[at] = bm[at - 1];
+          bi[at] = bi[at - 1];
+          at--;
+        }
+        bd[at] = d2;
+        bm[at] = dmax;
+        bi[at] = j;
+        m += m < k;
+      }
+    });
+  cnt = min(m, k);
   // the widening searches, from the k nearest
   int jm[kMax];
   int jmax = 0;
-  for (int i = 0; i < cnt; i++)
+  for (int e = 0; e < cnt; e++)
   {
-    double dmax;
-    const double d2 = re_d2(R.pos + 3 * (long long)R.tg[bi[i]], q, R, dmax);
-    jm[i] = re_jmin(d2, dmax, radii, n_radii);
-    jmax = max(jmax, jm[i]);
+    jm[e] = re_jmin(bd[e], bm[e], radii, n_radii);
+    jmax = max(jmax, jm[e]);
+    bi[e] = __float_as_int(R.raw[bi[e]].w); // the packed tracer
   }
   const int to_find = min(nt, k);
   int J = jmax;

@@ -167,7 +167,7 @@ enum Slot
   S_PR_SH, S_PR_SCR, S_PR_POS, S_PR_MASS, S_PR_ORD, S_PR_NB, S_PR_MBND, S_PR_MBP, S_PR_OUTF, S_PR_OUTI, S_PR_OUTL,
   S_RE_OFF, S_RE_SG, S_RE_GP, S_RE_FL, S_RE_RK, S_RE_TG, S_RE_TS, S_RE_GO, S_RE_POS, S_RE_TY, S_RE_DEST,
   S_SET_LIST, S_SET_NODES, S_SET_KEY, S_SET_VAL, S_SET_XCH, S_SET_TOT,
-  S_RE_QK, S_RE_QKA, S_RE_QV, S_RE_QVA,
+  S_RE_RAW, S_RE_QK, S_RE_QKA, S_RE_QV, S_RE_QVA,
   S_NUM
 };
 
@@ -1366,8 +1366,10 @@ int reassign_run(hbtg_handle *H, const hbtg_params *p, const hbtg_reassign *r, i
                        *qkey_alt = P.get<unsigned long long>(S_RE_QKA, (size_t)nq);
     Q.qkey = qkey;
     Q.qval = qval;
+    Q.raw = P.get<float4>(S_RE_RAW, t1);
+    k_re_leaves<<<blocks_for(src_total, 256), 256, 0, st>>>(Q, D, src_total);
     k_re_queries<<<blocks_for(N, 256), 256, 0, st>>>(Q, D, N);
-    launches++;
+    launches += 2;
     if (radix_sort_pairs<unsigned long long>(qkey, qval, qkey_alt, qval_alt, nq, 0, 3 * kReDigits + bits,
                                              mem.radix_table(nq), mem.radix_scan_scratch(nq), st, &launches,
                                              H->ticket))
