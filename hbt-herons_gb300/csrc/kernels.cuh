@@ -389,23 +389,41 @@ __device__ __forceinline__ void root_axis(double lo, double hi, double len, floa
   kp[d] = (float)o;
   kp[3 + d] = (float)(o - (double)(float)o);
 }
+// floor(log2 q) for q > 0 is its exponent, except that a double logarithm
+// rounds up to the next integer when q is a few ulps below a power of two:
+// there the logarithm itself is taken.  (It and a loop of halvings made
+// k_root 13 us on 900 subhaloes, now 9: FP64 has a long latency here.)
+__device__ __forceinline__ double floor_log2(double q)
+{
+  const long long u = __double_as_longlong(q);
+  if ((u & 0xfffffffffffffll) > 0xffffffffff000ll || u < (1ll << 52))
+    return floor(log2(q));
+  return (double)(int)((u >> 52) - 1023);
+}
 __device__ __forceinline__ void root_levels(double len, const KParams &K, float *kp)
 {
   kp[6] = len > 0. ? (float)(2097152.0 / len) : 0.f;
   int exact_levels = 21;
   if (K.res > 0.f && len > 0.)
   {
-    const double lv = floor(log2(len / (double)K.res)) + 2.;
+    const double lv = floor_log2(len / (double)K.res) + 2.;
     exact_levels = lv < 1. ? 1 : (lv > 21. ? 21 : (int)lv);
   }
   kp[7] = __int_as_float(exact_levels);
 }
-// A cell at level L has side len * 2^-min(L, kstar) (src/gravity_tree.cpp:38-42).
+// A cell at level L has side len * 2^-min(L, kstar) (src/gravity_tree.cpp:38-42):
+// kstar halvings take len below the resolution, counted from the exponents
+// (both are doubles of floats, so never subnormal).
 __device__ __forceinline__ void root_sides(double len, const KParams &K, float *kp)
 {
   int kstar = 0;
-  for (double l = len; l >= (double)K.res && kstar < 1000; l *= 0.5)
-    kstar++;
+  if (len >= (double)K.res)
+  {
+    const long long l = __double_as_longlong(len), r = __double_as_longlong((double)K.res);
+    const long long frac = 0xfffffffffffffll;
+    kstar = K.res > 0.f ? (int)(l >> 52) - (int)(r >> 52) + ((l & frac) >= (r & frac) ? 1 : 0) : 1000;
+    kstar = min(kstar, 1000);
+  }
   kp[8] = __int_as_float(kstar);
   kp[11] = (float)len;
 }
@@ -1615,7 +1633,8 @@ __device__ __forceinline__ float com_offset(float x, float o, float m, const KPa
 // (src/subhalo_unbind.cpp:151-198).  Each thread sums 16 consecutive items
 // with compensated float partials (FP64 is scarce on this GPU); the partials
 // are added in double.  Offsets that need the periodic wrap are formed in
-// double as the reference does.
+// double as the reference does.  (Four items' loads in flight per thread, at
+// 78 registers: 102 us where this takes 95, 3.3e6 items.)
 __global__ void k_com(DevState D, KParams K, int total)
 {
   const int ipt = D.com_ipt;
@@ -1701,22 +1720,45 @@ __global__ void k_com(DevState D, KParams K, int total)
 
 // Frame and bound mass from the k_com sums of subhalo s
 // (CentreOfMassReferenceFrame, src/subhalo_unbind.cpp:151-198).
-__device__ void frame_from_sums(DevState &D, const KParams &K, int s)
+// The whole warp calls it, each lane with its subhalo (take: whether it has
+// one): the partials of a subhalo with many are added by all its lanes (one
+// after another they held k_control at 18 us on a halo of 1e5, now 10).
+__device__ void frame_from_sums(DevState &D, const KParams &K, int s, bool take)
 {
   double c[7];
   for (int q = 0; q < 7; q++)
-    c[q] = D.com[7 * s + q];
+    c[q] = take ? D.com[7 * s + q] : 0.;
   // add the partials of the k_com blocks lying entirely inside this subhalo
   // (same test as k_com: the block's item range [b0, b1) lies in [lo, hi))
   const long long per_block = 256LL * D.com_ipt;
-  const long long lo = D.fin_off[s], hi = D.fin_off[s + 1], total = D.fin_off[D.S];
-  for (long long b = (lo + per_block - 1) / per_block; b * per_block < hi; b++)
-  {
-    const long long b1 = min(total, (b + 1) * per_block);
-    if (b1 <= hi)
+  const long long lo = take ? D.fin_off[s] : 0, hi = take ? D.fin_off[s + 1] : 0, total = D.fin_off[D.S];
+  int b0 = (int)((lo + per_block - 1) / per_block), b1 = (int)(hi == total ? (hi + per_block - 1) / per_block : hi / per_block);
+  const bool many = b1 - b0 > 4;
+  if (!many)
+    for (int b = b0; b < b1; b++)
       for (int q = 0; q < 7; q++)
-        c[q] += D.com_part[7 * b + q];
+        c[q] += D.com_part[7LL * b + q];
+  const int lane = threadIdx.x & 31;
+  for (unsigned left = __ballot_sync(0xffffffffu, many); left; left &= left - 1u)
+  {
+    const int src = __ffs(left) - 1;
+    const int f = __shfl_sync(0xffffffffu, b0, src), e = __shfl_sync(0xffffffffu, b1, src);
+    double v[7] = {0., 0., 0., 0., 0., 0., 0.};
+    for (int b = f + lane; b < e; b += kWarp)
+#pragma unroll
+      for (int q = 0; q < 7; q++)
+        v[q] += D.com_part[7LL * b + q];
+#pragma unroll
+    for (int q = 0; q < 7; q++)
+    {
+      for (int o = 16; o > 0; o >>= 1)
+        v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+      if (lane == src)
+        c[q] += v[q];
+    }
   }
+  if (!take)
+    return;
   const double M = c[0];
   const float4 o = D.pm[D.ord[D.off[s]]];
   const double org[3] = {o.x, o.y, o.z};
@@ -1735,9 +1777,10 @@ __device__ void frame_from_sums(DevState &D, const KParams &K, int s)
 __global__ void k_control(DevState D, KParams K)
 {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.S || D.state[s] != kActive)
+  const bool take = s < D.S && D.state[s] == kActive;
+  frame_from_sums(D, K, s, take);
+  if (!take)
     return;
-  frame_from_sums(D, K, s);
   const int nb = D.nbound[s];
   if ((float)nb >= __fmul_rn((float)D.nlast[s], K.bmp))
     D.state[s] = kConverged;

@@ -363,8 +363,8 @@ constexpr int kRadixItems = 8;
 constexpr int kRadixTile = kRadixThreads * kRadixItems;
 
 // Sorts of at most this many tiles (of 2048 items) scan their digit table in
-// the histogram kernel: its last block adds up the digits (a thread each,
-// tile by tile) and writes every tile's first output slot per digit.  Two
+// the histogram kernel: its last block adds up the digits and writes every
+// tile's first output slot per digit.  Two
 // launches a pass instead of five: a call on one halo of 1e5
 // particles (28 passes) takes 2.63 ms instead of 2.82.  Above, one block's trip
 // over the table costs more than the launches.
@@ -395,13 +395,34 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const K *__restric
   table[blockIdx.x * 256 + threadIdx.x] = cnt[threadIdx.x];
   if (!last_block(ticket))
     return;
-  __shared__ int wsum[kRadixThreads / kWarp];
+  // the last block: each warp takes an eighth of the tiles, each lane eight digits of them
+  constexpr int kWarps = kRadixThreads / kWarp;
+  __shared__ int part[kWarps][256];
+  __shared__ int wsum[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int *col = table + threadIdx.x; // this thread's digit
-  int total = 0;
+  const int per = (tiles + kWarps - 1) / kWarps, t0 = warp * per, t1 = min(tiles, t0 + per);
+  int4 *rows = reinterpret_cast<int4 *>(table) + 2 * lane; // 64 int4 a tile
+  int4 a = make_int4(0, 0, 0, 0), b = a;
+  auto add4 = [](int4 &x, const int4 &y) {
+    x.x += y.x;
+    x.y += y.y;
+    x.z += y.z;
+    x.w += y.w;
+  };
 #pragma unroll 8
-  for (int t = 0; t < tiles; t++)
-    total += __ldcg(col + 256 * t);
+  for (int t = t0; t < t1; t++)
+  {
+    add4(a, __ldcg(rows + 64 * t));
+    add4(b, __ldcg(rows + 64 * t + 1));
+  }
+  reinterpret_cast<int4 *>(part[warp])[2 * lane] = a;
+  reinterpret_cast<int4 *>(part[warp])[2 * lane + 1] = b;
+  __syncthreads();
+  // digits in order, each warp's tiles in order (a thread per digit)
+  int total = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; w++)
+    total += part[w][threadIdx.x];
   const int incl = warp_inclusive_scan(total, lane);
   if (lane == 31)
     wsum[warp] = incl;
@@ -409,18 +430,34 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const K *__restric
   int run = incl - total;
   for (int w = 0; w < warp; w++)
     run += wsum[w];
-  for (int t0 = 0; t0 < tiles; t0 += 8)
+#pragma unroll
+  for (int w = 0; w < kWarps; w++)
   {
-    int c[8];
+    const int c = part[w][threadIdx.x];
+    part[w][threadIdx.x] = run;
+    run += c;
+  }
+  __syncthreads();
+  a = reinterpret_cast<int4 *>(part[warp])[2 * lane];
+  b = reinterpret_cast<int4 *>(part[warp])[2 * lane + 1];
+  for (int t = t0; t < t1; t += 4)
+  {
+    int4 x[4], y[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++)
-      c[k] = t0 + k < tiles ? __ldcg(col + 256 * (t0 + k)) : 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (t0 + k < tiles)
+    for (int k = 0; k < 4; k++)
+      if (t + k < t1)
       {
-        col[256 * (t0 + k)] = run;
-        run += c[k];
+        x[k] = __ldcg(rows + 64 * (t + k));
+        y[k] = __ldcg(rows + 64 * (t + k) + 1);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (t + k < t1)
+      {
+        rows[64 * (t + k)] = a;
+        rows[64 * (t + k) + 1] = b;
+        add4(a, x[k]);
+        add4(b, y[k]);
       }
   }
 }

@@ -459,10 +459,10 @@ __global__ void k_warm_scatter(DevState D, int join_uncertain)
 __global__ void k_frame_flagged(DevState D, KParams K, int clear)
 {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.S || !D.flag_s[s])
+  const bool flagged = s < D.S && D.flag_s[s];
+  frame_from_sums(D, K, s, flagged && D.fin_off[s + 1] > D.fin_off[s]);
+  if (!flagged)
     return;
-  if (D.fin_off[s + 1] > D.fin_off[s])
-    frame_from_sums(D, K, s);
   if (clear)
     D.flag_s[s] = 0;
 }
