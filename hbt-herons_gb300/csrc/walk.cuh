@@ -411,10 +411,35 @@ __device__ __forceinline__ float near_term(float nm, float r2, const KParams &K,
 {
   if (__any_sync(0xffffffffu, r2 < h2s))
     return softened_term(-nm, r2, K, h2);
-  return nm * rsqrt_normal(r2);
+  return __fmul_rn(nm, rsqrt_normal(r2));
+}
+
+// Squared distances of a pair of wrapped entries with flags f (wrap_axis).
+__device__ __forceinline__ float2 pair_r2_wrapped(const float4 &A, const float4 &B, uint2 f, float tx, float ty, float tz,
+                                                  const KParams &K)
+{
+  float r[2];
+#pragma unroll
+  for (int e = 0; e < 2; e++)
+  {
+    const unsigned fe = e ? f.y : f.x;
+    const float ex = e ? A.y : A.x, ey = e ? A.w : A.z, ez = e ? B.y : B.x;
+    if (fe & kMixed)
+      r[e] = dist2(sep<true>(ex, tx, K), sep<true>(ey, ty, K), sep<true>(ez, tz, K));
+    else
+      r[e] = dist2(__fsub_rn(ex, (fe & 1u) ? __fsub_rn(tx, K.box) : tx),
+                   __fsub_rn(ey, (fe & 2u) ? __fsub_rn(ty, K.box) : ty),
+                   __fsub_rn(ez, (fe & 4u) ? __fsub_rn(tz, K.box) : tz));
+  }
+  return make_float2(r[0], r[1]);
 }
 
 // Near list: the softened kernel where r < h (src/gravity_tree.cpp:150-162).
+// Near entries are those within h of the targets' box, so most eights of them
+// lie beyond h of every target itself: one vote settles that for the eight,
+// and their terms need no branch each (with a vote and a branch per entry a
+// near entry took 280 cycles of its warp on a 5e6-particle plain batch, a
+// masked far one 45; now 208, and 99 instead of 190 on a subsampled one).
 // With Wrap, `flags` holds how the targets take each entry (wrap_axis).
 template <bool Wrap>
 __device__ __forceinline__ void eval_near(const float4 *ea, const float4 *eb, const unsigned *mask,
@@ -425,41 +450,40 @@ __device__ __forceinline__ void eval_near(const float4 *ea, const float4 *eb, co
   const uint2 *nm2 = reinterpret_cast<const uint2 *>(mask), *nf2 = reinterpret_cast<const uint2 *>(flags);
   for (int i = 0; i < n; i += 8)
   {
-    float part = 0.f;
-#pragma unroll 1
+    float r2[8], nm[8];
+#pragma unroll
     for (int q = 0; q < 4; q++)
     {
       const int pp = (i >> 1) + q;
       const float4 A = ea[pp], B = eb[pp];
       const uint2 mk = nm2[pp];
-      float2 r2;
+      float2 r;
       if (Wrap)
       {
         const uint2 f = nf2[pp];
-        if ((f.x | f.y) == 0u)
-          r2 = pair_r2(A, B, ntx, nty, ntz);
-        else
-        {
-          float r[2];
-#pragma unroll
-          for (int e = 0; e < 2; e++)
-          {
-            const unsigned fe = e ? f.y : f.x;
-            const float ex = e ? A.y : A.x, ey = e ? A.w : A.z, ez = e ? B.y : B.x;
-            if (fe & kMixed)
-              r[e] = dist2(sep<true>(ex, tx, K), sep<true>(ey, ty, K), sep<true>(ez, tz, K));
-            else
-              r[e] = dist2(__fsub_rn(ex, (fe & 1u) ? __fsub_rn(tx, K.box) : tx),
-                           __fsub_rn(ey, (fe & 2u) ? __fsub_rn(ty, K.box) : ty),
-                           __fsub_rn(ez, (fe & 4u) ? __fsub_rn(tz, K.box) : tz));
-          }
-          r2 = make_float2(r[0], r[1]);
-        }
+        r = (f.x | f.y) == 0u ? pair_r2(A, B, ntx, nty, ntz) : pair_r2_wrapped(A, B, f, tx, ty, tz, K);
       }
       else
-        r2 = pair_r2(A, B, ntx, nty, ntz);
-      part += near_term((mk.x & lanebit) ? B.z : 0.f, r2.x, K, h2, h2s);
-      part += near_term((mk.y & lanebit) ? B.w : 0.f, r2.y, K, h2, h2s);
+        r = pair_r2(A, B, ntx, nty, ntz);
+      r2[2 * q] = r.x;
+      r2[2 * q + 1] = r.y;
+      nm[2 * q] = (mk.x & lanebit) ? B.z : 0.f;
+      nm[2 * q + 1] = (mk.y & lanebit) ? B.w : 0.f;
+    }
+    const float least = fminf(fminf(fminf(r2[0], r2[1]), fminf(r2[2], r2[3])),
+                              fminf(fminf(r2[4], r2[5]), fminf(r2[6], r2[7])));
+    float part = 0.f;
+    if (__any_sync(0xffffffffu, least < h2s))
+    {
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        part = __fadd_rn(part, near_term(nm[q], r2[q], K, h2, h2s));
+    }
+    else
+    {
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        part = __fadd_rn(part, __fmul_rn(nm[q], rsqrt_normal(r2[q])));
     }
     kahan_add(sum, comp, part);
   }
