@@ -47,8 +47,8 @@ constexpr int kSettleSlots = 8192;  // tree slots of a block (each block of a cl
 constexpr int kSettleCluster = 8;   // blocks of a cluster's team
 constexpr int kGrid = 0;            // team size standing for the whole (cooperative) grid
 // Targets up to which one block takes a subhalo (a chunk of 32 per warp, or
-// four when there are more of that size than clusters), and a cluster; above,
-// the grid: its barriers cost most (some 3 us), and it takes one subhalo at a
+// four in the correction loop or when there are more of that size than
+// clusters), and a cluster; above, the grid: its barriers cost most (some 3 us), and it takes one subhalo at a
 // time.  One of 46,000 particles with 50 iterations left took 34 ms with a
 // cluster's 64 warps, 31 ms in lock step and 19 ms with the grid.
 constexpr int kSettleSmall = 256, kSettleOne = 1024, kSettleMid = 8192;
@@ -98,7 +98,8 @@ __global__ void k_settle_pick(DevState D, KParams K, SettleArgs A)
   const bool sampled = !D.corr[s] && K.max_sample > 0 && !(n < K.max_sample + D.nunsample[s]);
   if (sampled || (D.corr[s] ? D.nlast[s] - n : n) > kSettleSrc)
     return;
-  const int c = n <= kSettleSmall ? kSettleA : n <= kSettleOne ? kSettleB : n <= kSettleMid ? kSettleC : kSettleD;
+  // (the correction loop's trees are small: a block's barriers are cheaper there than a cluster's warps)
+  const int c = n <= kSettleSmall || (n <= kSettleOne && D.corr[s]) ? kSettleA : n <= kSettleOne ? kSettleB : n <= kSettleMid ? kSettleC : kSettleD;
   A.list[(size_t)c * D.S + atomicAdd(&A.count[c], 1)] = s;
 }
 
@@ -342,6 +343,15 @@ __device__ __forceinline__ bool settle_tree(const DevState &D, const KParams &K,
   if (lane == 0 && mine)
     atomicOr(levels, mine);
   __syncthreads();
+  // A small tree is built in shared memory, where the unsorted keys were, and
+  // copied out whole: its levels follow one another with shared memory's latency
+  // instead of L2's (with the sums below kept in pairs: a 1e6-particle
+  // subsampled call 11.5 -> 11.2 ms).
+  const int slots = m + 2 * cells;
+  float4 *const out = T;
+  const bool small = slots < kSettleSrc * (int)sizeof(t.key[0]) / (int)sizeof(float4); // and the padding slot
+  if (small)
+    T = reinterpret_cast<float4 *>(t.key);
   // slots in preorder (k_tree_emit)
   for (int i = tid; i < m; i += kSettleThreads)
   {
@@ -393,6 +403,9 @@ __device__ __forceinline__ bool settle_tree(const DevState &D, const KParams &K,
     }
     __syncthreads();
   }
+  if (small)
+    for (int i = tid; i < slots; i += kSettleThreads)
+      out[i] = T[i];
   return true;
 }
 
@@ -648,11 +661,12 @@ __global__ void __launch_bounds__(kSettleThreads, 3) k_settle(DevState D, KParam
 #pragma unroll
         for (int c = 0; c < 7; c++)
         {
-          double v = acc[c].value();
+          PairSum v = acc[c];
+#pragma unroll
           for (int h = 16; h > 0; h >>= 1)
-            v += __shfl_xor_sync(0xffffffffu, v, h);
+            v.add(PairSum{__shfl_xor_sync(0xffffffffu, v.hi, h), __shfl_xor_sync(0xffffffffu, v.lo, h)});
           if (lane == 0)
-            dsum[w][c] = v;
+            dsum[w][c] = v.value();
         }
         __syncthreads();
         if (tid < 7)
