@@ -339,24 +339,17 @@ struct IterationDriver
     mem.mark(1);
   }
 
-  // Blocks of the grid's team: all must be resident.
-  int settle_grid()
-  {
-    const int smem = (int)sizeof(SettleShared);
-    int per_sm = 0;
-    mem.check(cudaFuncSetAttribute(k_settle<kGrid>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    mem.check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_settle<kGrid>, kSettleThreads, (size_t)smem));
-    return std::min(kSettleMaxBlocks, sm_count * std::max(1, std::min(per_sm, kSettleGridPerSm)));
-  }
+  // Blocks of the grid's team, one per SM: all are resident.
+  int settle_grid() const { return std::min(kSettleMaxBlocks, sm_count); }
 
   template <int C>
   void launch_settle(int blocks)
   {
-    const int smem = (int)sizeof(SettleShared);
+    const int smem = (int)sizeof(SettleShared<C>);
     mem.check(cudaFuncSetAttribute(k_settle<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(kSettleThreads);
+    cfg.blockDim = dim3((unsigned)settle_threads(C));
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

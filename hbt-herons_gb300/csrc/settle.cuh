@@ -41,19 +41,20 @@ namespace hbtg
 namespace
 {
 
-constexpr int kSettleThreads = 256, kSettleWarps = kSettleThreads / kWarp;
+// Threads of a block (C: blocks of its team).  The grid's blocks are one per
+// SM, with enough warps for a chunk of 32 targets each.
+constexpr int kGrid = 0; // team size standing for the whole (cooperative) grid
+__host__ __device__ constexpr int settle_threads(int C) { return C == kGrid ? 512 : 256; }
 constexpr int kSettleSrc = 2048;    // tree sources of a team
 constexpr int kSettleSlots = 8192;  // tree slots of a block (each block of a cluster builds the tree for itself)
 constexpr int kSettleCluster = 8;   // blocks of a cluster's team
-constexpr int kGrid = 0;            // team size standing for the whole (cooperative) grid
 // Targets up to which one block takes a subhalo (a chunk of 32 per warp, or
 // four in the correction loop or when there are more of that size than
 // clusters), and a cluster; above, the grid: its barriers cost most (some 3 us), and it takes one subhalo at a
 // time.  One of 46,000 particles with 50 iterations left took 34 ms with a
-// cluster's 64 warps, 31 ms in lock step and 19 ms with the grid.
+// cluster's 64 warps, 31 ms in lock step and 15 ms with the grid.
 constexpr int kSettleSmall = 256, kSettleOne = 1024, kSettleMid = 8192;
 constexpr int kSettleTeams1 = 456, kSettleTeams8 = 38; // most teams of one launch (3 blocks fit an SM)
-constexpr int kSettleGridPerSm = 2;                     // blocks per SM of the grid's team
 constexpr int kSettleMaxBlocks = 1024;                  // of a team (the grid's)
 enum SettleClass : int
 {
@@ -81,11 +82,23 @@ struct SettleTree
   int X[kSettleSrc];               // cells before each item
   unsigned short levels[kSettleSrc]; // first level of its cells | their number << 8
 };
-union SettleShared
+template <int C>
+union SettleWork
 {
   SettleTree t;
-  WalkWarp walk[kSettleWarps];
+  WalkWarp walk[settle_threads(C) / kWarp];
   uint32_t tail[kSettleSrc];
+};
+// A block of a larger team has the shared memory of its SM to itself and keeps
+// its tree there, for the multipoles and for the walk: with both in L2 they
+// took 108 and 77 us of an iteration of the grid over 35,000 particles with
+// 1,000 tree sources, and a call with 50 of those 41.5 ms instead of 35.0.
+constexpr int kSettleOwn = 4096; // slots
+template <int C>
+struct SettleShared
+{
+  SettleWork<C> u;
+  float4 nodes[C == 1 ? 1 : kSettleOwn];
 };
 
 // Subhaloes that a team can take over at the top of an iteration.
@@ -119,7 +132,8 @@ __device__ __forceinline__ void team_sync()
 
 // Exclusive scan of one int per thread of the block; `par` alternates between
 // two sets of partial sums, so one barrier is enough.
-__device__ __forceinline__ int block_scan(int v, int (*part)[kSettleWarps], int &par, int &total)
+template <int Warps>
+__device__ __forceinline__ int block_scan(int v, int (*part)[Warps], int &par, int &total)
 {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int incl = warp_inclusive_scan(v, lane);
@@ -129,7 +143,7 @@ __device__ __forceinline__ int block_scan(int v, int (*part)[kSettleWarps], int 
   int before = 0;
   total = 0;
 #pragma unroll
-  for (int k = 0; k < kSettleWarps; k++)
+  for (int k = 0; k < Warps; k++)
   {
     const int c = part[par][k];
     before += k < w ? c : 0;
@@ -197,16 +211,18 @@ __device__ __forceinline__ void team_counts(int &c0, int &c1, int &base, int blo
   xpar ^= 1;
 }
 
-// Tree of the m sources at ord[0..m) in shared memory t and slots T: false
-// when it does not fit.  Returns its root cube's side and, in t.sval, the
+// Tree of the m sources at ord[0..m), by way of the arrays t, in the slots T or
+// (T changed) the block's own: false when it does not fit.  Returns its root cube's side and, in t.sval, the
 // sources in key order.  Every block of a team builds the same tree; of
 // several, each ranks a share of the sources and they exchange the order.
 template <int C>
 __device__ __forceinline__ bool settle_tree(const DevState &D, const KParams &K, const SettleArgs &A, const int *ord,
-                                            int m, SettleTree &t, float4 *T, int team, int rank, int blocks, double *root,
-                                            float *kp, unsigned (*red)[6], int (*part)[kSettleWarps], int &par,
-                                            unsigned *levels, int &cells)
+                                            int m, SettleTree &t, float4 *own, float4 *&T, int team, int rank, int blocks,
+                                            double *root, float *kp, unsigned (*red)[6],
+                                            int (*part)[settle_threads(C) / kWarp], int &par, unsigned *levels,
+                                            int &cells)
 {
+  constexpr int kSettleThreads = settle_threads(C), kSettleWarps = kSettleThreads / kWarp;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   // bounding box (k_bbox)
   unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
@@ -343,15 +359,18 @@ __device__ __forceinline__ bool settle_tree(const DevState &D, const KParams &K,
   if (lane == 0 && mine)
     atomicOr(levels, mine);
   __syncthreads();
-  // A small tree is built in shared memory, where the unsorted keys were, and
-  // copied out whole: its levels follow one another with shared memory's latency
-  // instead of L2's (with the sums below kept in pairs: a 1e6-particle
-  // subsampled call 11.5 -> 11.2 ms).
-  const int slots = m + 2 * cells;
+  // One block builds a small tree in shared memory, where the unsorted keys
+  // were, and copies it out whole: its levels follow one another with shared
+  // memory's latency instead of L2's (with the sums below kept in pairs: a
+  // 1e6-particle subsampled call 11.5 -> 11.2 ms).  Of a larger team each block
+  // keeps it (T) in its own shared memory where it fits.
+  const int slots = m + 2 * cells; // and a padding slot
   float4 *const out = T;
-  const bool small = slots < kSettleSrc * (int)sizeof(t.key[0]) / (int)sizeof(float4); // and the padding slot
+  const bool small = C == 1 && slots < kSettleSrc * (int)sizeof(t.key[0]) / (int)sizeof(float4);
   if (small)
     T = reinterpret_cast<float4 *>(t.key);
+  else if (C != 1 && slots < kSettleOwn)
+    T = own;
   // slots in preorder (k_tree_emit)
   for (int i = tid; i < m; i += kSettleThreads)
   {
@@ -404,16 +423,21 @@ __device__ __forceinline__ bool settle_tree(const DevState &D, const KParams &K,
     __syncthreads();
   }
   if (small)
+  {
     for (int i = tid; i < slots; i += kSettleThreads)
       out[i] = T[i];
+    T = out;
+  }
   return true;
 }
 
 template <int C>
-__global__ void __launch_bounds__(kSettleThreads, 3) k_settle(DevState D, KParams K, SettleArgs A)
+__global__ void __launch_bounds__(settle_threads(C), C == 1 ? 3 : 1) k_settle(DevState D, KParams K, SettleArgs A)
 {
+  constexpr int kSettleThreads = settle_threads(C), kSettleWarps = kSettleThreads / kWarp;
   extern __shared__ __align__(16) unsigned char settle_smem[];
-  SettleShared &U = *reinterpret_cast<SettleShared *>(settle_smem);
+  SettleShared<C> &SH = *reinterpret_cast<SettleShared<C> *>(settle_smem);
+  SettleWork<C> &U = SH.u;
   __shared__ double root[4], dsum[kSettleWarps][7], dtot[7];
   __shared__ float kp[12], rp[3], rv[3], op[3], ov[3], s_mbound;
   __shared__ unsigned red[kSettleWarps][6], levels;
@@ -426,7 +450,7 @@ __global__ void __launch_bounds__(kSettleThreads, 3) k_settle(DevState D, KParam
   const bool b_large = A.count[kSettleB] <= kSettleTeams8; // class B to the clusters
   const int c0 = C == 1 ? kSettleA : C == kGrid ? kSettleD : kSettleC;
   const int n0 = A.count[c0], n1 = C != kGrid && b_large == (C > 1) ? A.count[kSettleB] : 0, count = n0 + n1;
-  float4 *T = A.nodes + (size_t)blockIdx.x * kSettleSlots;
+  float4 *const slots = A.nodes + (size_t)blockIdx.x * kSettleSlots;
   double *xch = A.xch + (size_t)team * 2 * blocks * 8;
   int par = 0, xpar = 0; // alternating halves of `part` / wcnt and of xch
   for (int q = team; q < count; q += teams)
@@ -454,8 +478,9 @@ __global__ void __launch_bounds__(kSettleThreads, 3) k_settle(DevState D, KParam
       if (m > kSettleSrc || (!corr && K.max_sample > 0 && !(n < K.max_sample + nuns)))
         break; // lock step goes on with it
       int cells = 0;
-      if (m > 0 && !settle_tree<C>(D, K, A, ord + (corr ? n : 0), m, U.t, T, team, rank, blocks, root, kp, red, part, par,
-                                   &levels, cells))
+      float4 *T = slots;
+      if (m > 0 && !settle_tree<C>(D, K, A, ord + (corr ? n : 0), m, U.t, SH.nodes, T, team, rank, blocks, root, kp, red,
+                                   part, par, &levels, cells))
         break;
       built += (unsigned long long)cells;
       iter++;

@@ -489,12 +489,12 @@ __device__ __forceinline__ void eval_near(const float4 *ea, const float4 *eb, co
   }
 }
 
-// A tree slot; Fresh: the tree may have been written by this kernel, so not
-// through the read-only path.
+// A tree slot; Fresh: the tree may have been written by this kernel, or lie in
+// shared memory, so not through the read-only path.
 template <bool Fresh>
 __device__ __forceinline__ float4 tree_slot(const float4 *p)
 {
-  return Fresh ? __ldca(p) : __ldg(p);
+  return Fresh ? *p : __ldg(p);
 }
 
 // The reference's stackless walk of one range [a, e) of sibling subtrees for
