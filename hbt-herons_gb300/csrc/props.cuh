@@ -40,6 +40,7 @@ struct PropState
   const float *mb_pos;       // [3S] most-bound positions (the profile's centre)
   int *cnt, *fin_off;        // [S+1] bound counts and their exclusive scan
   float *rr, *mm;            // [T] distance and mass of each item
+  int *seg;                  // [T] its subhalo (the sort keeps the packing, so also that of each sorted item)
   uint32_t *k32, *val, *k32_alt, *val_alt;
   double *mcum;              // [T] cumulative mass in sorted order
   unsigned long long *vkey;  // [S] packed (v, ~rank) of the largest v = M(<r)/r
@@ -137,6 +138,7 @@ __global__ void __launch_bounds__(256) k_prop_items(PropState P, int total)
       P.mm[j] = m;
       P.k32[j] = __float_as_uint(rr); // r >= 0: the bits order as the values
       P.val[j] = (uint32_t)j;
+      P.seg[j] = s;
     }
     float dx = __fsub_rn(x[0], c[0]), dy = __fsub_rn(x[1], c[1]), dz = __fsub_rn(x[2], c[2]);
     if (P.periodic)
@@ -187,7 +189,7 @@ __global__ void k_prop_segkeys(PropState P, const uint32_t *__restrict__ v, uint
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < total)
-    k[i] = (uint32_t)find_segment<int>(P.fin_off, P.S, (int)v[i]);
+    k[i] = (uint32_t)P.seg[v[i]];
 }
 
 struct PropMassLoad
@@ -196,8 +198,7 @@ struct PropMassLoad
   const uint32_t *sorted;
   __device__ SegD operator()(long long i) const
   {
-    const int s = find_segment<int>(P.fin_off, P.S, (int)i);
-    return SegD{(double)P.mm[sorted[i]], i == P.fin_off[s] ? 1 : 0};
+    return SegD{(double)P.mm[sorted[i]], i == 0 || P.seg[i] != P.seg[i - 1] ? 1 : 0};
   }
 };
 struct PropMassStore
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(256) k_prop_profile(PropState P, const uint32_
   {
     const long long ii = first + r * kWarp + lane;
     const int i = (int)min(ii, (long long)total - 1);
-    const int s = find_segment_warp(P.fin_off, P.S, i);
+    const int s = P.seg[i];
     const int s0 = __shfl_sync(0xffffffffu, s, 0);
     const bool one = __shfl_sync(0xffffffffu, s, 31) == s0;
     const int q = i - P.fin_off[s];

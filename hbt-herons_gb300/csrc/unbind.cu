@@ -163,7 +163,7 @@ enum Slot
   S_NODES, S_TABLE, S_SCRATCH, S_CELLS, S_LVL, S_COUNTER, S_PERM, S_PERMA, S_FBL, S_FBC, S_TMASS, S_COMP, S_SP, S_TGT, S_BND, S_FACTOR,
   S_WARMI, S_REF0, S_RMAX, S_MMAX, S_WBB, S_HIST, S_TAB, S_FEAT, S_PROP, S_PNB, S_PEN, S_MODEL, S_NB1,
   S_POTI, S_WCTR, S_FRAMEW, S_TUNE,
-  S_PR_OFF, S_PR_CNT, S_PR_FIN, S_PR_RR, S_PR_MM, S_PR_K, S_PR_V, S_PR_KA, S_PR_VA, S_PR_MC, S_PR_VK, S_PR_SO,
+  S_PR_OFF, S_PR_CNT, S_PR_FIN, S_PR_RR, S_PR_MM, S_PR_SEG, S_PR_K, S_PR_V, S_PR_KA, S_PR_VA, S_PR_MC, S_PR_VK, S_PR_SO,
   S_PR_SH, S_PR_SCR, S_PR_POS, S_PR_MASS, S_PR_ORD, S_PR_NB, S_PR_MBND, S_PR_MBP, S_PR_OUTF, S_PR_OUTI, S_PR_OUTL,
   S_RE_OFF, S_RE_SG, S_RE_GP, S_RE_FL, S_RE_RK, S_RE_TG, S_RE_TS, S_RE_GO, S_RE_POS, S_RE_TY, S_RE_DEST,
   S_SET_LIST, S_SET_NODES, S_SET_KEY, S_SET_VAL, S_SET_XCH, S_SET_TOT,
@@ -1100,6 +1100,7 @@ int props_run(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, int sna
   const size_t t1 = (size_t)std::max(T, 1);
   Q.rr = P.get<float>(S_PR_RR, t1);
   Q.mm = P.get<float>(S_PR_MM, t1);
+  Q.seg = P.get<int>(S_PR_SEG, t1);
   Q.k32 = P.get<uint32_t>(S_PR_K, t1);
   Q.val = P.get<uint32_t>(S_PR_V, t1);
   Q.k32_alt = P.get<uint32_t>(S_PR_KA, t1);
