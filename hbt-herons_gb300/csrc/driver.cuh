@@ -517,14 +517,21 @@ struct IterationDriver
                                                                                                         fin_total);
       launches++;
     }
-    k_epilogue<<<sb, 256, 0, st>>>(D, K, O);
+    OutPtrs scalars = O;
+    if (O.core && S <= kCoreWarps)
+    {
+      k_epi_core<<<grid_for((long long)S * kWarp, 128), 128, 0, st>>>(D, K, O.core);
+      launches++;
+      scalars.core = nullptr;
+    }
+    k_epilogue<<<sb, 256, 0, st>>>(D, K, scalars);
     if (O.mbound_type)
     {
       if (K.dm_only)
         mem.check(cudaMemsetAsync(O.mbound_type, 0, sizeof(float) * 6 * (size_t)S, st));
       else
       {
-        k_type_masses<<<grid_for(S, 8), 256, 0, st>>>(D, O.mbound_type);
+        k_type_masses<<<grid_for(S, kTypeWarps), 32 * kTypeWarps, 0, st>>>(D, O.mbound_type);
         launches++;
       }
     }

@@ -1976,7 +1976,7 @@ __device__ __forceinline__ int units_in_binade(int type, const int (&ty)[kTypeRo
     if (r >= row0 && r < row0 + rows && ty[r] == type)
     {
       const float x = __fmul_rn(m[r], inv), i = rintf(x); // m / u, exact
-      ok = ok && x >= 0.f && x < 65536.f && fabsf(x - i) != 0.5f; // < 2^16 each: 2048 of them fit an int
+      ok = ok && x >= 0.f && x < 1048576.f && fabsf(x - i) != 0.5f; // < 2^20 each: a warp's 256 stay below 2^28
       q += ok ? (int)i : 0;
     }
   return q;
@@ -2029,29 +2029,30 @@ __device__ __forceinline__ void add_type_rows(float &sum, int type, const int (&
 
 // MboundType as CountParticleTypes sums it (src/subhalo.cpp:311-393): per
 // type, float additions in bound order, by integer sums within a binade
-// (above).  A block takes eight subhaloes: each warp one of at most
-// kTypeLong bound particles, 256 at a time, then the whole block each longer
-// one, 2048 at a time; only where a type's sum leaves its binade (once per
-// doubling) do the warps add their 256 in turn, and one row of 32 particle by
-// particle.  Bound by the longest subhalo's chain of steps: one warp replaying
-// every addition took 5.3 of the 29.0 ms of a 4e6-particle hydro call (largest
-// subhalo 1.7e5 particles); one warp per subhalo by 256 made that call 26.4
-// ms, blocks by 2048 25.1 ms.  The line at 2048 is where one block step
-// replaces eight warp steps.
-constexpr int kTypeLong = 2048;
-__global__ void __launch_bounds__(256) k_type_masses(DevState D, float *out)
+// (above).  A block takes eight subhaloes, a grid apart (so that long neighbours
+// go to different blocks): each warp one of at most kTypeLong bound particles,
+// 256 at a time, then the whole block each longer one, 2048 at a time.  Where
+// a type's sum leaves its binade (once per doubling), the warps before the
+// crossing still count in one step, the one that crosses adds its 256 row by
+// row, and the rest count in the next binade.  Bound by the longest subhalo's
+// chain of steps: one warp replaying every addition took 5.3 of the 29.0 ms of
+// a 4e6-particle hydro call (largest subhalo 1.7e5 particles), the warps in
+// turn at every crossing 0.77 ms, this 0.47 ms (0.52 in blocks of 512 threads,
+// 0.58 of 1024: fewer subhaloes at a time on an SM).
+constexpr int kTypeLong = 2048, kTypeWarps = 8;
+__global__ void __launch_bounds__(32 * kTypeWarps) k_type_masses(DevState D, float *out)
 {
-  __shared__ int s_units[2][8][6];
-  __shared__ int s_bad[2][6]; // bit w: warp w's masses of the type want the slow way
+  __shared__ int s_units[kTypeWarps]; // a warp's units of one type; negative: its masses want the slow way
   __shared__ float s_sum[6];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int s_first = blockIdx.x * 8;
   auto bound = [&](int s) {
     const int st = s < D.S ? D.state[s] : (int)kEmpty;
     return (st == kConverged || st == kMaxIter) ? D.nbound[s] : 0;
   };
-  auto load = [&](const int *ord, int nb, int i0, int (&t)[kTypeRows], float (&m)[kTypeRows]) {
+  int ty[kTypeRows], nty[kTypeRows];
+  float m[kTypeRows], nm[kTypeRows];
+  auto load = [&](const int *ord, int nb, int i0) { // into nty, nm
     int p[kTypeRows];
 #pragma unroll
     for (int r = 0; r < kTypeRows; r++)
@@ -2062,12 +2063,10 @@ __global__ void __launch_bounds__(256) k_type_masses(DevState D, float *out)
 #pragma unroll
     for (int r = 0; r < kTypeRows; r++)
     {
-      t[r] = p[r] >= 0 ? D.ty[p[r]] & 7 : 7;
-      m[r] = p[r] >= 0 ? D.pm[p[r]].w : 0.f;
+      nty[r] = p[r] >= 0 ? D.ty[p[r]] & 7 : 7;
+      nm[r] = p[r] >= 0 ? D.pm[p[r]].w : 0.f;
     }
   };
-  int ty[kTypeRows], nty[kTypeRows];
-  float m[kTypeRows], nm[kTypeRows];
   auto next = [&]() {
 #pragma unroll
     for (int r = 0; r < kTypeRows; r++)
@@ -2076,27 +2075,29 @@ __global__ void __launch_bounds__(256) k_type_masses(DevState D, float *out)
       m[r] = nm[r];
     }
   };
+  auto types = [&]() { // bit t: the warp's rows hold type t (bit 7: past the end)
+    unsigned has = 0u;
+#pragma unroll
+    for (int r = 0; r < kTypeRows; r++)
+      has |= 1u << ty[r];
+    return __reduce_or_sync(full, has);
+  };
   { // one subhalo per warp
-    const int s = s_first + w, nb = bound(s);
+    const int s = blockIdx.x + w * gridDim.x, nb = bound(s);
     if (s < D.S && nb <= kTypeLong)
     {
       const int *ord = D.ord + D.off[s];
       float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}; // the same on every lane
-      load(ord, nb, 0, ty, m);
+      load(ord, nb, 0);
       for (int i0 = 0; i0 < nb; i0 += kTypeRows * kWarp)
       {
-        load(ord, nb, i0 + kTypeRows * kWarp, nty, nm);
+        next();
+        load(ord, nb, i0 + kTypeRows * kWarp);
+        const unsigned has = types();
 #pragma unroll
         for (int t = 0; t < 6; t++)
-        {
-          bool has = false;
-#pragma unroll
-          for (int r = 0; r < kTypeRows; r++)
-            has = has || ty[r] == t;
-          if (__any_sync(full, has))
+          if (has & (1u << t))
             add_type_rows(sum[t], t, ty, m);
-        }
-        next();
       }
       float v = sum[0];
 #pragma unroll
@@ -2106,92 +2107,154 @@ __global__ void __launch_bounds__(256) k_type_masses(DevState D, float *out)
         out[6 * s + lane] = v;
     }
   }
-  for (int k = 0; k < 8; k++)
+  for (int k = 0; k < kTypeWarps; k++)
   { // the long ones, by the whole block
-    const int s = s_first + k, nb = bound(s);
+    const int s = blockIdx.x + k * gridDim.x, nb = bound(s);
     if (nb <= kTypeLong)
       continue;
     const int *ord = D.ord + D.off[s];
     __syncthreads(); // s_sum of the subhalo before has been written out
     if (threadIdx.x < 6)
-    {
       s_sum[threadIdx.x] = 0.f;
-      s_bad[0][threadIdx.x] = 0;
-    }
-    __syncthreads();
-    load(ord, nb, w * kTypeRows * kWarp, ty, m);
-    int par = 0;
-    for (int i0 = 0; i0 < nb; i0 += 256 * kTypeRows, par ^= 1)
+    load(ord, nb, w * kTypeRows * kWarp);
+    for (int i0 = 0; i0 < nb; i0 += kTypeWarps * kTypeRows * kWarp)
     {
-      load(ord, nb, i0 + 256 * kTypeRows + w * kTypeRows * kWarp, nty, nm);
-#pragma unroll
-      for (int t = 0; t < 6; t++)
-      {
-        float inv;
-        unsigned A;
-        bool ok = sum_binade(s_sum[t], inv, A);
-        bool any = false;
-#pragma unroll
-        for (int r = 0; r < kTypeRows; r++)
-          any = any || ty[r] == t;
-        int q = 0;
-        if (__any_sync(full, any))
-        {
-          q = units_in_binade(t, ty, m, 0, kTypeRows, inv, ok);
-          q = __reduce_add_sync(full, q);
-          if (!__all_sync(full, ok) && lane == 0)
-            atomicOr(&s_bad[par][t], 1 << w);
-        }
-        if (lane == 0)
-          s_units[par][w][t] = q;
-      }
-      __syncthreads();
-      unsigned slow = 0u; // types that want the slow way; the same on every thread
-      float sum[6];
-#pragma unroll
-      for (int t = 0; t < 6; t++)
-      {
-        sum[t] = s_sum[t];
-        float inv;
-        unsigned A;
-        sum_binade(sum[t], inv, A);
-        int q = 0;
-#pragma unroll
-        for (int v = 0; v < 8; v++)
-          q += s_units[par][v][t];
-        if (s_bad[par][t] || !add_units(sum[t], A, q))
-          slow |= 1u << t;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0)
-      {
-#pragma unroll
-        for (int t = 0; t < 6; t++)
-          if (!(slow & (1u << t)))
-            s_sum[t] = sum[t];
-      }
-      if (threadIdx.x < 6)
-        s_bad[par ^ 1][threadIdx.x] = 0;
-      for (int v = 0; slow && v < 8; v++)
-      { // the warps in turn
-        __syncthreads();
-        if (w == v)
-#pragma unroll
-          for (int t = 0; t < 6; t++)
-            if (slow & (1u << t))
-            {
-              float a = s_sum[t];
-              add_type_rows(a, t, ty, m);
-              if (lane == 0)
-                s_sum[t] = a;
-            }
-      }
-      __syncthreads();
       next();
+      load(ord, nb, i0 + (kTypeWarps + w) * kTypeRows * kWarp);
+      const unsigned has = types();
+#pragma unroll 1
+      for (int t = 0; t < 6; t++)
+      {
+        if (__syncthreads_or((int)(has & (1u << t))) == 0)
+          continue; // the block holds none of the type
+        for (int from = 0; from < kTypeWarps;)
+        { // the warps from `from` on, up to the first that cannot be counted in this binade
+          float sum = s_sum[t], inv;
+          unsigned A;
+          bool ok = sum_binade(sum, inv, A);
+          int q = 0;
+          if (has & (1u << t))
+          {
+            q = ok ? units_in_binade(t, ty, m, 0, kTypeRows, inv, ok) : 0;
+            q = __reduce_add_sync(full, q);
+            if (!__all_sync(full, ok))
+              q = -1;
+          }
+          if (lane == 0)
+            s_units[w] = q;
+          __syncthreads();
+          // every warp: the prefix of the warps' units, and the first that stops it
+          const int u = lane >= from && lane < kTypeWarps ? s_units[lane] : 0;
+          const unsigned bad = __ballot_sync(full, u < 0);
+          const int incl = warp_inclusive_scan(min(max(u, 0), 0x1000000), lane); // 2^24 leaves any binade
+          const unsigned over = __ballot_sync(full, A + (unsigned)incl >= 0x1000000u);
+          const unsigned stop = (bad | over) & (full << from) & (full >> (32 - kTypeWarps));
+          const int first = stop ? __ffs(stop) - 1 : kTypeWarps;
+          const int Q = first > 0 ? __shfl_sync(full, incl, first - 1) : 0;
+          if (first > from && Q > 0)
+            add_units(sum, A, Q);
+          __syncthreads(); // s_sum and s_units have been read
+          if (first < kTypeWarps ? w == first : threadIdx.x < 32)
+          {
+            if (first < kTypeWarps)
+              add_type_rows(sum, t, ty, m);
+            if (lane == 0)
+              s_sum[t] = sum;
+          }
+          __syncthreads();
+          from = first + 1;
+        }
+      }
     }
     if (threadIdx.x < 6)
       out[6 * s + threadIdx.x] = s_sum[threadIdx.x];
   }
+}
+
+// The core phase-space properties (GetCorePhaseSpaceProperties,
+// src/subhalo_merge.cpp:94-181) from their sums: mass, first and second
+// moments of position (about org) and velocity.
+__device__ __forceinline__ void put_core(float *cr, double msum, const double *ps, const double *ps2, const double *vs,
+                                         const double *vs2, const double *org, const KParams &K)
+{
+  double sr = 0., sv = 0.;
+  for (int d = 0; d < 3; d++)
+  {
+    const double p = ps[d] / msum, v = vs[d] / msum;
+    float cp = (float)p;
+    if (K.periodic)
+      cp = (float)((double)cp + org[d]);
+    cr[d] = cp;
+    cr[3 + d] = (float)v;
+    sr += ps2[d] / msum - p * p;
+    sv += vs2[d] / msum - v * v;
+  }
+  cr[6] = (float)sqrt(sr);
+  cr[7] = (float)sqrt(sv);
+}
+
+// The same by a warp per subhalo, its lanes 32 bound particles at a time, for
+// calls on at most kCoreWarps subhaloes: one thread's chain of loads and FP64
+// operations over the twenty particles of a core was 40 of k_epilogue's 55 us,
+// and most of a call's latency has nothing beside it.  With more subhaloes a
+// thread each does the same work with fewer FP64 instructions.
+constexpr int kCoreWarps = 4096;
+__global__ void k_epi_core(DevState D, KParams K, float *core)
+{
+  const int s = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (s >= D.S) // whole warps
+    return;
+  const int st = D.state[s];
+  const int nb = (st == kConverged || st == kMaxIter) ? D.nbound[s] : 0;
+  float *cr = core + 8 * s;
+  if (nb == 0)
+  {
+    if (lane < 8)
+      cr[lane] = lane < 3 ? D.mb_pos[3 * s + lane] : lane < 6 ? D.mb_vel[3 * s + lane - 3] : 0.f;
+    return;
+  }
+  const int *ord = D.ord + D.off[s];
+  const long long core_size = max((long long)((float)nb * K.core_factor), K.core_min);
+  const float4 x0 = D.pm[ord[0]];
+  const double org[3] = {K.periodic ? (double)x0.x : 0., K.periodic ? (double)x0.y : 0., K.periodic ? (double)x0.z : 0.};
+  double q[13]; // mass, then first and second moments of position and velocity
+  for (int k = 0; k < 13; k++)
+    q[k] = 0.;
+  long long used = 0;
+  for (int pass = 0; pass < 2 && used != core_size; pass++)
+    for (int i0 = 0; i0 < nb && used != core_size; i0 += kWarp)
+    { // first the tracers, then the others
+      const int p = i0 + lane < nb ? ord[i0 + lane] : -1;
+      const bool mine = p >= 0 && is_tracer_bits(D.ty[p]) == (pass == 0);
+      const unsigned all = __ballot_sync(0xffffffffu, mine);
+      const long long at = used + __popc(all & ((1u << lane) - 1u));
+      if (mine && at < core_size)
+      {
+        const float4 x = D.pm[p], v = D.vu[p];
+        const double m = x.w;
+        q[0] += m;
+        const float xs[3] = {x.x, x.y, x.z}, vv[3] = {v.x, v.y, v.z};
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+        {
+          double dx = xs[d];
+          if (K.periodic)
+            dx = nearest_d(dx - org[d], K.half, K.box);
+          const double dv = vv[d];
+          q[1 + d] += m * dx;
+          q[4 + d] += m * dx * dx;
+          q[7 + d] += m * dv;
+          q[10 + d] += m * dv * dv;
+        }
+      }
+      used = min(core_size, used + (long long)__popc(all));
+    }
+#pragma unroll
+  for (int k = 0; k < 13; k++)
+    for (int o = 16; o > 0; o >>= 1)
+      q[k] += __shfl_xor_sync(0xffffffffu, q[k], o);
+  if (lane == 0)
+    put_core(cr, q[0], q + 1, q + 4, q + 7, q + 10, org, K);
 }
 
 // Scalar outputs of each subhalo (one thread per subhalo): kinematics, type
@@ -2304,22 +2367,7 @@ __global__ void k_epilogue(DevState D, KParams K, OutPtrs O)
       if (used == core_size)
         break;
     }
-  for (int d = 0; d < 3; d++)
-  {
-    ps[d] /= msum;
-    ps2[d] /= msum;
-    float cp = (float)ps[d];
-    if (K.periodic)
-      cp = (float)((double)cp + org[d]);
-    cr[d] = cp;
-    ps2[d] -= ps[d] * ps[d];
-    vs[d] /= msum;
-    vs2[d] /= msum;
-    cr[3 + d] = (float)vs[d];
-    vs2[d] -= vs[d] * vs[d];
-  }
-  cr[6] = (float)sqrt(ps2[0] + ps2[1] + ps2[2]);
-  cr[7] = (float)sqrt(vs2[0] + vs2[1] + vs2[2]);
+  put_core(cr, msum, ps, ps2, vs, vs2, org, K);
 }
 
 } // namespace
