@@ -45,6 +45,53 @@ __global__ void k_pot_repack(DevState D, const float *__restrict__ pos, const fl
   }
 }
 
+// What the host reports of a call, added up on the device (one small copy in
+// place of per-subhalo arrays).
+struct CallTotals
+{
+  unsigned long long bound;        // sum of nbound
+  int max_iter;                    // some subhalo stopped at max_iterations
+  int warm, restarts;              // warm-started subhaloes, those restarted cold
+  int settle_most;                 // most iterations of a team (settle.cuh) and the tree cells of all
+  unsigned long long settle_cells;
+};
+__global__ void k_call_totals(int S, const long long *nbound, const int *status, const int *warm,
+                              const unsigned long long *cells, const int *most, CallTotals *t)
+{
+  unsigned long long bound = 0;
+  int mi = 0, w = 0, r = 0;
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x)
+  {
+    bound += (unsigned long long)nbound[s];
+    mi |= status[s] == HBTG_SUB_MAX_ITER;
+    if (warm)
+    {
+      w += warm[s] != 0;
+      r += warm[s] == 2;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    bound += __shfl_xor_sync(0xffffffffu, bound, o);
+  mi = __reduce_or_sync(0xffffffffu, mi);
+  w = __reduce_add_sync(0xffffffffu, w);
+  r = __reduce_add_sync(0xffffffffu, r);
+  if ((threadIdx.x & 31) == 0)
+  {
+    atomicAdd(&t->bound, bound);
+    if (mi)
+      atomicOr(&t->max_iter, 1);
+    if (w)
+      atomicAdd(&t->warm, w);
+    if (r)
+      atomicAdd(&t->restarts, r);
+  }
+  if (cells && blockIdx.x == 0 && threadIdx.x == 0)
+  {
+    t->settle_cells = *cells;
+    t->settle_most = *most;
+  }
+}
+
 // One "subhalo" whose every particle is a source; the walk takes the
 // requested particles as targets (tgt list) with their self terms.
 __global__ void k_pot_plan(DevState D, int n_tgt, int phase)
@@ -166,7 +213,7 @@ enum Slot
   S_PR_OFF, S_PR_CNT, S_PR_FIN, S_PR_RR, S_PR_MM, S_PR_SEG, S_PR_K, S_PR_V, S_PR_KA, S_PR_VA, S_PR_MC, S_PR_VK, S_PR_SO,
   S_PR_SH, S_PR_SCR, S_PR_POS, S_PR_MASS, S_PR_ORD, S_PR_NB, S_PR_MBND, S_PR_MBP, S_PR_OUTF, S_PR_OUTI, S_PR_OUTL,
   S_RE_OFF, S_RE_SG, S_RE_GP, S_RE_FL, S_RE_RK, S_RE_TG, S_RE_TS, S_RE_GO, S_RE_POS, S_RE_TY, S_RE_DEST,
-  S_SET_LIST, S_SET_NODES, S_SET_KEY, S_SET_VAL, S_SET_XCH, S_SET_TOT,
+  S_TOTALS, S_STAGE, S_SET_LIST, S_SET_NODES, S_SET_KEY, S_SET_VAL, S_SET_XCH, S_SET_TOT,
   S_RE_RAW, S_RE_QK, S_RE_QKA, S_RE_QV, S_RE_QVA,
   S_NUM
 };
@@ -219,6 +266,12 @@ inline unsigned blocks_for(long long n, int threads)
 
 } // namespace
 
+// Host-pointer calls whose arrays take at most this much go through one pinned
+// buffer and one copy each way: some thirty copies of a few hundred bytes were
+// 0.2 ms of a 0.65 ms call on one subhalo of 300 particles (now 0.47 ms).
+// Above, copying the arrays on the host first would cost more than that.
+constexpr size_t kStageBytes = 256 * 1024;
+
 struct hbtg_handle
 {
   int device = 0;
@@ -229,6 +282,8 @@ struct hbtg_handle
   cudaEvent_t copy_events[7] = {};          // host-pointer calls: copy phases and the side streams
   cudaEvent_t epilogue_wait = nullptr;      // set for one call: the epilogue waits for this event
   Pool pool;
+  cudaEvent_t span[2] = {};                 // first and last event of a call
+  void *stage = nullptr;                    // pinned staging of small host-pointer calls, then of the totals
   unsigned *ticket = nullptr;               // a device zero for the last-block scans (primitives.cuh)
   hbtg_stats stats{};
   bool count_interactions = false;
@@ -352,6 +407,7 @@ struct PoolMem
                                                              256LL * 4096)));
   }
   unsigned *ticket() { return H->ticket; }
+  unsigned long long *warm_totals() { return H->pool.get<unsigned long long>(S_SET_TOT, 2 + kSettleClasses); }
   int *cell_list(long long cells) { return H->pool.get<int>(S_CELLS, (size_t)std::max<long long>(cells, 1)); }
   int *level_counts() { return H->pool.get<int>(S_LVL, 2 * kLevels); }
   float4 *tree_slots(long long slots)
@@ -419,9 +475,7 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
   H->stats.n_particles = N;
   if (S == 0)
     return HBTG_OK;
-  cudaEvent_t t0, t1;
-  HBTG_CUDA(cudaEventCreate(&t0));
-  HBTG_CUDA(cudaEventCreate(&t1));
+  const cudaEvent_t t0 = H->span[0], t1 = H->span[1];
   HBTG_CUDA(cudaEventRecord(t0, st));
 
   PoolMem mem{H, st, {}};
@@ -553,8 +607,6 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
       if (wa->features_only)
       {
         HBTG_CUDA(cudaStreamSynchronize(st));
-        cudaEventDestroy(t0);
-        cudaEventDestroy(t1);
         H->stats.kernel_launches = R.launches;
         return HBTG_OK;
       }
@@ -571,14 +623,6 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
       W.prop = prop;
     }
     warm_run(R, W, wc, !wa->proposal);
-    std::vector<int> warm(S);
-    HBTG_CUDA(cudaMemcpyAsync(warm.data(), D.warm, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-    HBTG_CUDA(cudaStreamSynchronize(st));
-    for (int s = 0; s < S; s++)
-    {
-      wc.warm_subhaloes += warm[s] != 0;
-      wc.restarts += warm[s] == 2;
-    }
   }
 
   OutPtrs O;
@@ -602,8 +646,19 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
   HBTG_CUDA(cudaMemcpyAsync(b->ref_vel, D.ref_vel, fbytes, cudaMemcpyDefault, st));
   HBTG_CUDA(cudaMemcpyAsync(b->mostbound_pos, D.mb_pos, fbytes, cudaMemcpyDefault, st));
   HBTG_CUDA(cudaMemcpyAsync(b->mostbound_vel, D.mb_vel, fbytes, cudaMemcpyDefault, st));
+  CallTotals *dt = P.get<CallTotals>(S_TOTALS, 1);
+  HBTG_CUDA(cudaMemsetAsync(dt, 0, sizeof(CallTotals), st));
+  const bool settled = R.settle_from >= 0;
+  k_call_totals<<<std::min(blocks_for(S, 256), (unsigned)(2 * H->sm_count)), 256, 0, st>>>(
+    S, O.nbound, O.status, D.warm, settled ? R.settle_args.cells : nullptr, R.settle_args.most, dt);
+  R.launches++;
+  R.check();
+  CallTotals *tot = reinterpret_cast<CallTotals *>(static_cast<unsigned char *>(H->stage) + kStageBytes);
+  HBTG_CUDA(cudaMemcpyAsync(tot, dt, sizeof(CallTotals), cudaMemcpyDeviceToHost, st));
   HBTG_CUDA(cudaEventRecord(t1, st));
   HBTG_CUDA(cudaEventSynchronize(t1));
+  wc.warm_subhaloes = tot->warm;
+  wc.restarts = tot->restarts;
   H->last_S = S;
   H->last_N = N;
   H->last_ord = D.ord;
@@ -628,8 +683,6 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
   H->stats.ms_final = phase_ms[5];
   float ms = 0.f;
   HBTG_CUDA(cudaEventElapsedTime(&ms, t0, t1));
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
   H->stats.ms_total = ms;
   H->stats.kernel_launches = R.launches;
   H->stats.walk_launches = R.walk_launches;
@@ -637,12 +690,10 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
   H->stats.walk_blocks_per_sm = R.walk_blocks_per_sm;
   H->stats.global_iterations = R.global_iter;
   H->stats.tree_nodes = R.tree_nodes;
-  if (R.settle_from >= 0)
+  if (settled)
   { // the teams' share
-    unsigned long long tot[2] = {};
-    HBTG_CUDA(cudaMemcpy(tot, R.settle_args.cells, sizeof(tot), cudaMemcpyDeviceToHost));
-    H->stats.tree_nodes += (int64_t)tot[0];
-    H->stats.global_iterations = std::max<int64_t>(R.global_iter, R.settle_from + (int)(tot[1] & 0xffffffffu));
+    H->stats.tree_nodes += (int64_t)tot->settle_cells;
+    H->stats.global_iterations = std::max<int64_t>(R.global_iter, R.settle_from + tot->settle_most);
   }
   if (H->count_interactions)
   {
@@ -659,19 +710,8 @@ int run_device(hbtg_handle *H, const hbtg_params *p, const hbtg_batch *b, cudaSt
     for (int q = 0; q < 8; q++)
       H->stats.walk_cycles[q] = (int64_t)c[8 + q];
   }
-  // summary counters
-  std::vector<long long> nb(S);
-  HBTG_CUDA(cudaMemcpy(nb.data(), b->nbound, sizeof(long long) * S, cudaMemcpyDeviceToHost));
-  long long tot = 0;
-  for (long long v : nb)
-    tot += v;
-  H->stats.total_bound = tot;
-  int any_max = 0;
-  std::vector<int> stv(S);
-  HBTG_CUDA(cudaMemcpy(stv.data(), b->status, sizeof(int) * S, cudaMemcpyDeviceToHost));
-  for (int v : stv)
-    any_max |= (v == HBTG_SUB_MAX_ITER);
-  return any_max ? HBTG_ERR_MAX_ITER : HBTG_OK;
+  H->stats.total_bound = (int64_t)tot->bound;
+  return tot->max_iter ? HBTG_ERR_MAX_ITER : HBTG_OK;
 }
 
 template <typename T>
@@ -735,6 +775,114 @@ struct HostCall
   const hbtg_prior *prior = nullptr; // host arrays
 };
 
+// Every host array of a batch: pointer in it, pointer in its device copy, size
+// and direction (pure inputs first, then in/out, then outputs).
+struct HostArray
+{
+  const void *host;
+  void **dev;
+  size_t bytes;
+  int dir; // 0 in, 1 in and out, 2 out
+};
+
+// A small host-pointer call through the handle's pinned buffer; false when it
+// does not fit.
+bool staged_call(HostCall &c, long long N, int &rc)
+{
+  hbtg_handle *H = c.H;
+  hbtg_batch *b = c.b;
+  const size_t S = (size_t)b->n_sub, n = (size_t)N;
+  hbtg_batch d = *b;
+  WarmArgs wa;
+  const void *nb_prev = c.learned && c.prior ? c.prior->nbound_prev : nullptr;
+  const void *e_prev = nb_prev ? c.prior->energy_prev : nullptr;
+  auto at = [](auto &p) { return reinterpret_cast<void **>(const_cast<void *>(static_cast<const void *>(&p))); };
+  const HostArray arr[] = {
+    {b->pos, at(d.pos), 12 * n, 0},
+    {b->vel, at(d.vel), 12 * n, 0},
+    {b->mass, at(d.mass), 4 * n, 0},
+    {c.p->thermal ? b->u : nullptr, at(d.u), 4 * n, 0},
+    {b->id, at(d.id), 8 * n, 0},
+    {c.p->dm_only ? nullptr : b->type, at(d.type), n, 0},
+    {nb_prev, at(wa.nb_prev), 8 * S, 0},
+    {e_prev, at(wa.e_prev), 4 * n, 0},
+    {b->ref_pos, at(d.ref_pos), 12 * S, 1},
+    {b->ref_vel, at(d.ref_vel), 12 * S, 1},
+    {b->mostbound_pos, at(d.mostbound_pos), 12 * S, 1},
+    {b->mostbound_vel, at(d.mostbound_vel), 12 * S, 1},
+    {b->most_bound_id, at(d.most_bound_id), 8 * S, 1},
+    {b->order, at(d.order), 8 * n, 2},
+    {b->nbound, at(d.nbound), 8 * S, 2},
+    {b->mbound, at(d.mbound), 4 * S, 2},
+    {b->nbound_type, at(d.nbound_type), 48 * S, 2},
+    {b->mbound_type, at(d.mbound_type), 24 * S, 2},
+    {b->tracer_index, at(d.tracer_index), 8 * S, 2},
+    {b->kinematics, at(d.kinematics), 20 * S, 2},
+    {b->core, at(d.core), 32 * S, 2},
+    {b->energy, at(d.energy), 4 * n, 2},
+    {b->potential, at(d.potential), 4 * n, 2},
+    {b->iterations, at(d.iterations), 4 * S, 2},
+    {b->status, at(d.status), 4 * S, 2},
+  };
+  auto room = [](const HostArray &a) { return a.host ? (a.bytes + 255) & ~(size_t)255 : 0; };
+  size_t all = 0;
+  for (const HostArray &a : arr)
+    all += room(a);
+  if (all > kStageBytes)
+    return false;
+  cudaStream_t st = H->stream;
+  unsigned char *dev = H->pool.get<unsigned char>(S_STAGE, kStageBytes), *pin = static_cast<unsigned char *>(H->stage);
+  size_t end = 0, in_end = 0, out0 = 0;
+  int64_t h2d = 0, d2h = 0;
+  for (const HostArray &a : arr)
+  {
+    *a.dev = a.host ? dev + end : nullptr;
+    if (a.host && a.dir < 2 && a.bytes)
+    {
+      std::memcpy(pin + end, a.host, a.bytes);
+      h2d += (int64_t)a.bytes;
+    }
+    if (a.host && a.dir > 0)
+      d2h += (int64_t)a.bytes;
+    if (a.dir == 0)
+      out0 = end + room(a);
+    end += room(a);
+    if (a.dir < 2)
+      in_end = end;
+  }
+  cudaEvent_t *ev = H->copy_events;
+  HBTG_CUDA(cudaEventRecord(ev[0], st));
+  HBTG_CUDA(cudaMemcpyAsync(dev, pin, in_end, cudaMemcpyHostToDevice, st));
+  HBTG_CUDA(cudaEventRecord(ev[1], st));
+  if (c.learned)
+  {
+    wa.min_n = H->min_particles;
+    wa.first_test = H->first_test;
+  }
+  rc = run_device(H, c.p, &d, st, c.learned ? &wa : nullptr);
+  if (rc != HBTG_OK && rc != HBTG_ERR_MAX_ITER)
+    return true;
+  HBTG_CUDA(cudaEventRecord(ev[2], st));
+  HBTG_CUDA(cudaMemcpyAsync(pin + out0, dev + out0, end - out0, cudaMemcpyDeviceToHost, st));
+  HBTG_CUDA(cudaEventRecord(ev[3], st));
+  HBTG_CUDA(cudaStreamSynchronize(st));
+  end = 0;
+  for (const HostArray &a : arr)
+  {
+    if (a.host && a.dir > 0 && a.bytes)
+      std::memcpy(const_cast<void *>(a.host), pin + end, a.bytes);
+    end += room(a);
+  }
+  H->stats.h2d_bytes = h2d;
+  H->stats.d2h_bytes = d2h;
+  float t_up = 0.f, t_down = 0.f;
+  HBTG_CUDA(cudaEventElapsedTime(&t_up, ev[0], ev[1]));
+  HBTG_CUDA(cudaEventElapsedTime(&t_down, ev[2], ev[3]));
+  H->stats.ms_h2d = t_up;
+  H->stats.ms_d2h = t_down;
+  return true;
+}
+
 int host_call(void *arg)
 {
   HostCall &c = *static_cast<HostCall *>(arg);
@@ -745,6 +893,8 @@ int host_call(void *arg)
   if (rc != HBTG_OK)
     return rc;
   HBTG_CUDA(cudaSetDevice(H->device));
+  if (staged_call(c, N, rc))
+    return rc;
   cudaStream_t st = H->stream;
   const size_t S = (size_t)b->n_sub;
   Pool &P = H->pool;
@@ -1547,6 +1697,18 @@ int hbtg_create(hbtg_handle **handle, int device)
       delete h;
       return HBTG_ERR_CUDA;
     }
+  for (auto &e : h->span)
+    if (cudaEventCreate(&e) != cudaSuccess)
+    {
+      delete h;
+      return HBTG_ERR_CUDA;
+    }
+  if (cudaMallocHost(&h->stage, kStageBytes + 256) != cudaSuccess)
+  {
+    cudaGetLastError();
+    delete h;
+    return HBTG_ERR_NOMEM;
+  }
   *handle = h;
   return HBTG_OK;
 }
@@ -1558,6 +1720,9 @@ int hbtg_destroy(hbtg_handle *h)
   cudaSetDevice(h->device);
   h->pool.release();
   cudaFree(h->ticket);
+  cudaFreeHost(h->stage);
+  for (auto &e : h->span)
+    cudaEventDestroy(e);
   for (auto &e : h->walk_events)
     cudaEventDestroy(e);
   for (auto &e : h->phase_events)

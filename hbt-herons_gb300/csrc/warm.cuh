@@ -679,6 +679,28 @@ __global__ void k_warm_fallback_particles(DevState D)
   }
 }
 
+// Particles left out, and subhaloes marked for a cold restart.
+__global__ void k_warm_totals(DevState D, unsigned long long *tot)
+{
+  unsigned long long left_out = 0;
+  int restart = 0;
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < D.S; s += gridDim.x * blockDim.x)
+  {
+    left_out += (unsigned long long)D.nexcl[s];
+    restart += D.warm[s] == 4;
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    left_out += __shfl_xor_sync(0xffffffffu, left_out, o);
+  restart = __reduce_add_sync(0xffffffffu, restart);
+  if ((threadIdx.x & 31) == 0)
+  {
+    if (left_out)
+      atomicAdd(tot, left_out);
+    if (restart)
+      atomicAdd(tot + 1, (unsigned long long)restart);
+  }
+}
+
 // Training trace, in input order: which = 1 marks the survivors of the first
 // iteration (positions [0, Nbound after it): later iterations only reorder
 // inside that range); which = 0 marks the set whose potential decided the
@@ -856,16 +878,18 @@ void warm_run(IterationDriver<Mem> &R, const WarmBufs &W, WarmCounters &C, bool 
     R.check();
   }
   long long restarts = 0;
-  { // left-out counts and the subhaloes marked for a cold restart, in one host read
-    std::vector<int> nex(S), wm(S);
-    R.mem.check(cudaMemcpyAsync(nex.data(), D.nexcl, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-    R.mem.check(cudaMemcpyAsync(wm.data(), D.warm, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
+  { // left-out particles and the subhaloes marked for a cold restart, in one host read
+    unsigned long long *tot = R.mem.warm_totals();
+    R.mem.check(cudaMemsetAsync(tot, 0, 2 * sizeof(*tot), st));
+    k_warm_totals<<<std::min(sb, 1024u), 256, 0, st>>>(D, tot);
+    R.launches++;
+    R.check();
+    unsigned long long h[2] = {};
+    R.mem.check(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, st));
     R.mem.check(cudaStreamSynchronize(st));
     R.host_syncs++;
-    for (int v : nex)
-      C.excluded += v;
-    for (int v : wm)
-      restarts += (v == 4);
+    C.excluded += (long long)h[0];
+    restarts = (long long)h[1];
   }
   if (W.first_test)
     flagged_frames(R); // the frame of the set the second iteration evaluates
