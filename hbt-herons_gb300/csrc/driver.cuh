@@ -420,9 +420,8 @@ struct IterationDriver
       mem.mark(1);
       if (part_total > 0)
       {
-        k_energy<<<grid_for(part_total, 256), 256, 0, st>>>(D, K, part_total);
-        k_part_flags<<<grid_for(part_total + 1, 256), 256, 0, st>>>(D, part_total);
-        launches += 2;
+        k_energy<<<grid_for(part_total + 1, 256), 256, 0, st>>>(D, K, part_total);
+        launches++;
         check();
         scan<int, false>(D.flags, D.F, part_total + 1, mem.scan_scratch(part_total + 1), st, &launches, mem.ticket());
         k_part_count<<<sb, 256, 0, st>>>(D);

@@ -533,6 +533,11 @@ __device__ __forceinline__ bool descent_key_fast(float4 x, const float *kp, unsi
   return true;
 }
 
+// The subhalo of each packed source, kept by k_keys for the kernels that
+// follow the sort (it permutes a subhalo's sources only): the array is free
+// until the correction targets are flagged.
+__device__ __forceinline__ int *src_seg(const DevState &D) { return D.F; }
+
 // Keys by the fast descent; the few items it cannot decide are appended to
 // fb_list and finished by k_keys_fallback, so no warp diverges into FP64.
 __global__ void k_keys(DevState D, int total)
@@ -547,6 +552,7 @@ __global__ void k_keys(DevState D, int total)
     need = !descent_key_fast(D.pm[p], D.keyp + 12 * s, key);
     D.key[j] = key;
     D.val[j] = (uint32_t)p;
+    src_seg(D)[j] = s;
   }
   const unsigned m = __ballot_sync(0xffffffffu, need);
   if (m)
@@ -863,7 +869,7 @@ __global__ void k_tree_count(DevState D, int total)
     hist[threadIdx.x] = 0;
   __syncthreads();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = find_segment_warp(D.src_off, D.S, min(j, total - 1));
+  const int s = j < total ? src_seg(D)[j] : 0;
   if (j == total)
     D.cnt[j] = 0;
   else if (j < total)
@@ -994,7 +1000,7 @@ __global__ void k_tree_emit(DevState D, KParams K, int total)
   __syncthreads();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   int lo = 0, c = 0, seg_end = 0, base = 0;
-  const int s = find_segment_warp(D.src_off, D.S, min(j, total - 1));
+  const int s = j < total ? src_seg(D)[j] : 0;
   if (j < total)
   {
     const int seg0 = D.src_off[s], m = D.src_cnt[s];
@@ -1360,33 +1366,30 @@ __device__ __forceinline__ float corrected_energy(float e, float4 x, float4 v, f
   return __fadd_rn(e, __fsub_rn(__fadd_rn(dot, dK), pot));
 }
 
+// Energies, and what the partition needs of each packed item: whether it stays
+// bound (flags, with a trailing zero for the scan) and its subhalo (part_seg: a
+// search over the offsets was most of what each of the partition's kernels did).
+__device__ __forceinline__ int *part_seg(const DevState &D) { return D.cnt; } // free between the tree build and the next
 __global__ void k_energy(DevState D, KParams K, int total)
 {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int s = find_segment_warp(D.part_off, D.S, min(j, total - 1));
   if (j >= total)
+  {
+    if (j == total)
+      D.flags[j] = 0;
     return;
+  }
   const int k = j - D.part_off[s];
   const int p = D.ord[D.off[s] + k];
   const float4 x = D.pm[p], v = D.vu[p];
   const float *rp = D.ref_pos + 3 * s, *rv = D.ref_vel + 3 * s;
-  D.Ep[p] = D.corr[s] ? corrected_energy(D.Ep[p], x, v, D.pot[p], D.old_pos + 3 * s, D.old_vel + 3 * s, rp, rv, K)
-                      : binding_energy(x, v, D.pot[p], rp, rv, K);
-}
-
-__global__ void k_part_flags(DevState D, int total)
-{
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = find_segment_warp(D.part_off, D.S, min(j, total - 1));
-  if (j > total)
-    return;
-  if (j == total)
-  {
-    D.flags[j] = 0;
-    return;
-  }
-  const int k = j - D.part_off[s];
-  D.flags[j] = D.Ep[D.ord[D.off[s] + k]] < 0.f ? 1 : 0;
+  const float e = D.corr[s]
+                    ? corrected_energy(D.Ep[p], x, v, D.pot[p], D.old_pos + 3 * s, D.old_vel + 3 * s, rp, rv, K)
+                    : binding_energy(x, v, D.pot[p], rp, rv, K);
+  D.Ep[p] = e;
+  D.flags[j] = e < 0.f ? 1 : 0;
+  part_seg(D)[j] = s;
 }
 
 __global__ void k_part_count(DevState D)
@@ -1402,9 +1405,8 @@ __global__ void k_part_scatter(DevState D, int total)
 {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = j < total;
-  int s = find_segment_warp(D.part_off, D.S, min(j, total - 1)), tracer = 0;
-  if (!valid)
-    s = -1;
+  const int s = valid ? part_seg(D)[j] : -1;
+  int tracer = 0;
   if (valid)
   {
     const int k = j - D.part_off[s];
@@ -1425,9 +1427,9 @@ __global__ void k_part_scatter(DevState D, int total)
 __global__ void k_part_copy(DevState D, int total)
 {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = find_segment_warp(D.part_off, D.S, min(j, total - 1));
   if (j >= total)
     return;
+  const int s = part_seg(D)[j];
   const long long g = D.off[s] + (j - D.part_off[s]);
   D.ord[g] = D.ord_tmp[g];
 }

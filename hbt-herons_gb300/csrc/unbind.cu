@@ -1059,6 +1059,7 @@ int pot_call(void *arg)
   D.fb_count = P.get<int>(S_FBC, 1);
   D.cnt = P.get<int>(S_CNT, n1 + 1);
   D.X = P.get<int>(S_X, n1 + 1);
+  D.F = P.get<int>(S_F, n1 + 1);
   D.nodes = P.get<float4>(S_NODES, n1 * 3);
   D.interactions = P.get<unsigned long long>(S_COUNTER, kWalkCounters);
   D.walk_ctr = P.get<unsigned>(S_WCTR, (size_t)std::max(H->sm_count, 1));
@@ -1495,6 +1496,7 @@ int reassign_run(hbtg_handle *H, const hbtg_params *p, const hbtg_reassign *r, i
   D.fb_count = P.get<int>(S_FBC, 1);
   D.cnt = P.get<int>(S_CNT, t1 + 1);
   D.X = P.get<int>(S_X, t1 + 1);
+  D.F = P.get<int>(S_F, t1 + 1);
   D.interactions = P.get<unsigned long long>(S_COUNTER, kWalkCounters);
   if (T > 0)
   {
