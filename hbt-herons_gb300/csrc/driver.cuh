@@ -223,7 +223,7 @@ struct IterationDriver
     D.nodes = mem.tree_slots((long long)src_total + 2LL * internal + 1);
     D.cell_list = mem.cell_list(internal);
     tree_nodes += internal;
-    k_tree_emit<<<grid_for(src_total, 128), 128, 0, st>>>(D, K, src_total);
+    k_tree_emit<<<grid_for(src_total, 256), 256, 0, st>>>(D, K, src_total);
     launches++;
     // cell multipoles (or bounding boxes) bottom-up, deepest level first: one
     // launch per level of many cells, one per run of levels of few
