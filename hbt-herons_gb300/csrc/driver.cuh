@@ -18,7 +18,7 @@
 //   float4 *tree_slots(long long slots)          tree storage (may throw when too large)
 //   void mark(int phase)                         phase boundary for timing (may be a no-op)
 //   static constexpr bool kTeams                 whether it has working buffers for k_settle (else lock step to the end)
-//   void settle_buffers(SettleArgs &, int S, int grid)  those buffers, for a grid's team of that many blocks
+//   bool settle_buffers(SettleArgs &, int S, int grid)  those buffers, for a grid's team of that many blocks (false: no room)
 #pragma once
 
 #include <algorithm>
@@ -60,6 +60,7 @@ struct IterationDriver
   int64_t tree_nodes = 0;
   int64_t host_syncs = 0; // stream synchronisations for host reads of device totals
   int global_iter = 0;
+  bool teams = true;    // false once there was no room for their buffers
   int settle_from = -1; // lock-step iterations before the first k_settle of the call (-1: none)
   SettleArgs settle_args{};
 
@@ -318,7 +319,11 @@ struct IterationDriver
   void settle(long long live)
   {
     SettleArgs &A = settle_args;
-    mem.settle_buffers(A, S, live > kSettleMid ? settle_grid() : 0);
+    if (!mem.settle_buffers(A, S, live > kSettleMid ? settle_grid() : 0))
+    {
+      teams = false;
+      return;
+    }
     if (settle_from < 0)
     {
       settle_from = global_iter;
@@ -387,7 +392,7 @@ struct IterationDriver
     for (;;)
     {
       if constexpr (Mem::kTeams)
-        if (live <= kComSmall && live > 0 && !K.count_interactions)
+        if (live <= kComSmall && live > 0 && teams && !K.count_interactions)
           settle(live);
       k_plan<<<sb, 256, 0, st>>>(D, K);
       launches++;

@@ -6,7 +6,8 @@
 // by device-side exclusive scans of per-subhalo counts (src_off, chunk_off,
 // part_off, ...).  A packed item j is mapped back to its subhalo by a search
 // over the packed offsets (warp-cooperative in the per-item kernels:
-// find_segment_warp).  FP64 throughput is low on this GPU (about 1/64 of
+// find_segment_warp), or read back where an earlier kernel of the iteration
+// kept it (src_seg, part_seg).  FP64 throughput is low on this GPU (about 1/64 of
 // FP32, and 64-bit integer/float conversions issue to the same pipe), so the
 // per-item kernels use FP32 and integer arithmetic, with error-free
 // transforms or fixed point where the reference accumulates in double.
@@ -2055,8 +2056,8 @@ __device__ __forceinline__ void add_type_rows(float &sum, int type, const int (&
 // row, and the rest count in the next binade.  Bound by the longest subhalo's
 // chain of steps: one warp replaying every addition took 5.3 of the 29.0 ms of
 // a 4e6-particle hydro call (largest subhalo 1.7e5 particles), the warps in
-// turn at every crossing 0.77 ms, this 0.47 ms (0.52 in blocks of 512 threads,
-// 0.58 of 1024: fewer subhaloes at a time on an SM).
+// turn at every crossing 0.8 ms, this 0.53 ms (blocks of 512 or 1024 threads,
+// with fewer subhaloes at a time on an SM, make the final phase 0.05 or 0.12 ms longer).
 constexpr int kTypeLong = 2048, kTypeWarps = 8;
 __global__ void __launch_bounds__(32 * kTypeWarps) k_type_masses(DevState D, float *out)
 {

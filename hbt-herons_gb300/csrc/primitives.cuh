@@ -364,9 +364,9 @@ constexpr int kRadixTile = kRadixThreads * kRadixItems;
 
 // Sorts of at most this many tiles (of 2048 items) scan their digit table in
 // the histogram kernel: its last block adds up the digits and writes every
-// tile's first output slot per digit.  Two
-// launches a pass instead of five: a call on one halo of 1e5
-// particles (28 passes) takes 2.63 ms instead of 2.82.  Above, one block's trip
+// tile's first output slot per digit.  Two launches a pass instead of five,
+// which took a call on one halo of 1e5 particles (28 passes) from 2.82 to 2.63
+// ms.  Above, one block's trip
 // over the table costs more than the launches.
 constexpr int kRadixFused = 128;
 

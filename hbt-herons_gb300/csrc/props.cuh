@@ -6,7 +6,8 @@
 //
 // The bound particles of every subhalo are packed (item j = bound position k
 // of subhalo s).  One pass computes each item's distance from the most-bound
-// particle and its shape terms (summed per subhalo in double); the items are
+// particle and its shape terms (summed per subhalo in float pairs, TwoSum, and
+// those in double); the items are
 // then sorted by distance within their subhalo (radix sort by distance, then
 // stably by subhalo), the cumulative masses come from one segmented scan in
 // double, and the profile quantities from per-subhalo reductions over the

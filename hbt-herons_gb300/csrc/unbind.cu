@@ -417,7 +417,9 @@ struct PoolMem
     return H->pool.get<float4>(S_NODES, (size_t)slots);
   }
   static constexpr bool kTeams = true;
-  void settle_buffers(SettleArgs &A, int S, int grid)
+  // False when there is no room for them: the call then goes on in lock step.
+  bool settle_buffers(SettleArgs &A, int S, int grid)
+  try
   {
     Pool &P = H->pool;
     const size_t teams8 = (size_t)std::min(S, kSettleTeams8),
@@ -431,6 +433,11 @@ struct PoolMem
     A.cells = tot;
     A.most = reinterpret_cast<int *>(tot + 1);
     A.count = reinterpret_cast<int *>(tot + 2);
+    return true;
+  }
+  catch (const NoMem &)
+  {
+    return false;
   }
   void mark(int phase)
   {

@@ -45,7 +45,6 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
-#include <vector>
 
 #include "common.cuh"
 #include "driver.cuh"
