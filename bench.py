@@ -435,11 +435,14 @@ def bench_gpu(args):
 
     # roofline of the dominant kernel (the tree walk) in the learned arm
     peak = measure_fp32_peak(local)
-    walk_ms_per_launch = warm["ms_walk"] / max(1, warm["walk_launches"])
+    # (per launch of a timed step: a counted one stays in lock step and so has
+    # more; the interactions and the time include the late iterations' teams)
+    walk_launches = max(1.0, warm["walk_launches"] / args.steps)
+    walk_ms_per_launch = warm["ms_walk"] / args.steps / walk_launches
     cw = warm["counted"]
-    flops_per_launch = cw["interactions"] * FLOPS_PER_INTERACTION / max(1, cw["walk_launches"])
+    flops_per_launch = cw["interactions"] * FLOPS_PER_INTERACTION / walk_launches
     achieved = flops_per_launch / (walk_ms_per_launch * 1e-3) / 1e12
-    traffic = _walk_traffic(cw)
+    traffic = _walk_traffic(cw["interactions"] / walk_launches)
     issue = _walk_issue()
 
     cpu = parity = None
@@ -680,7 +683,7 @@ def _walk_issue():
         return json.load(f).get("issue_active_pct")
 
 
-def _walk_traffic(counted):
+def _walk_traffic(interactions_per_launch):
     """DRAM bytes per walk launch from the committed ncu summary of k_walk,
     scaled from the captured case to this one by interactions per launch."""
     path = os.path.join(HERE, "profiles", "k_walk_traffic.json")
@@ -689,7 +692,7 @@ def _walk_traffic(counted):
     with open(path) as f:
         d = json.load(f)
     per_interaction = d["dram_bytes_per_launch"] / max(1.0, d["interactions_per_launch"])
-    return per_interaction * counted["interactions"] / max(1, counted["walk_launches"])
+    return per_interaction * interactions_per_launch
 
 
 def main():
