@@ -126,6 +126,19 @@ __device__ __forceinline__ void mma_k64(float (&d)[4], const uint32_t (&a)[4][4]
   }
 }
 
+// sum += A B, the product by itself and the sum in one rounded FP32 addition:
+// added up inside the tensor core's accumulator, whose additions are not rounded to nearest, the
+// gradient drifts with the number of rows (error of dW1 against 64 bits 9e-6 of its norm at
+// 1e6 rows and 1e-4 at 8e6; so 3.5e-7 and 2.6e-7).
+__device__ __forceinline__ void mma_add(float (&sum)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  mma_bf16(d, a, b0, b1);
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    sum[q] += d[q];
+}
+
 // Forward pass of one 16-row tile.  g = lane / 4 (row), c = lane % 4.
 // Keeps the post-ReLU activations h1/h2 (FP32, C layout), their BF16 A
 // fragments, and the logits of rows g and g+8 (valid in every lane).
@@ -503,11 +516,11 @@ constexpr size_t kBwdSmemBytes = sizeof(BwdSmem);
 // A block takes 128 rows at a time, 16 per warp: forward, deltas, and H1,
 // dZ2, dZ1 and X staged as BF16 in shared memory.  The weight gradients are
 // then products over the 128 rows, each warp one slice of them (16 x 32 of
-// dW2, 8 columns of dW1) in register accumulators that stay from tile to
-// tile, as do each lane's bias and output-layer sums; a block adds its totals
+// dW2, 8 columns of dW1), 16 rows a product, added up in registers from tile to
+// tile, as are each lane's bias and output-layer sums; a block adds its totals
 // to the global gradient once, at the end.  Bound by latency: 65,536 rows are
 // four tiles per SM.  With a shared-memory atomic per weight and 16 rows
-// (4096 of them) the same call took 93.9 us, now 26.8 us.
+// (4096 of them) the same call took 93.9 us, now 28.2 us.
 __global__ void __launch_bounds__(kBwdWarps * 32, 1) k_mlp_backward(const float *__restrict__ w,
                                                                     const float *__restrict__ x,
                                                                     const float *__restrict__ y,
@@ -599,20 +612,20 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 1) k_mlp_backward(const float 
     *reinterpret_cast<uint32_t *>(&st.x[r0 + g + 8][2 * c + 8]) = 0u;
     __syncthreads();
     // dW2[i][j] = sum_r H1[r][i] dZ2[r][j]; dW1[k][j] = sum_r X[r][k] dZ1[r][j]
-#pragma unroll
+#pragma unroll 4 // whole, with the sums beside the products, it spills
     for (int k0 = 0; k0 < kBwdRows; k0 += 16)
     {
       uint32_t a[4], b[4];
       ldsm4<true>(a, &st.h1[k0 + ka][16 * mt + ca]);
       ldsm4<true>(b, &st.dz2[k0 + kbr][8 * nt0 + cb]);
-      mma_bf16(aw2[0], a, b[0], b[1]);
-      mma_bf16(aw2[1], a, b[2], b[3]);
+      mma_add(aw2[0], a, b[0], b[1]);
+      mma_add(aw2[1], a, b[2], b[3]);
       ldsm4<true>(b, &st.dz2[k0 + kbr][8 * nt0 + 16 + cb]);
-      mma_bf16(aw2[2], a, b[0], b[1]);
-      mma_bf16(aw2[3], a, b[2], b[3]);
+      mma_add(aw2[2], a, b[0], b[1]);
+      mma_add(aw2[3], a, b[2], b[3]);
       ldsm4<true>(a, &st.x[k0 + ka][ca]);
       ldsm4<true>(b, &st.dz1[k0 + kbr][16 * (wi >> 1) + cb]); // columns of two warps; this one's half
-      mma_bf16(aw1, a, (wi & 1) ? b[2] : b[0], (wi & 1) ? b[3] : b[1]);
+      mma_add(aw1, a, (wi & 1) ? b[2] : b[0], (wi & 1) ? b[3] : b[1]);
     }
     __syncthreads();
   }
