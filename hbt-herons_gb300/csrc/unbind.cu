@@ -23,6 +23,7 @@ int hbtg_mlp_propose(const float *weights, const float *features, uint8_t *prop,
 #include "driver.cuh"
 #include "props.cuh"
 #include "reassign.cuh"
+#include "resources.cuh"
 #include "kernels.cuh"
 #include "primitives.cuh"
 #include "warm.cuh"
@@ -266,28 +267,14 @@ inline unsigned blocks_for(long long n, int threads)
 
 } // namespace
 
-// Host-pointer calls whose arrays take at most this much go through one pinned
-// buffer and one copy each way: some thirty copies of a few hundred bytes were
-// 0.2 ms of a 0.65 ms call on one subhalo of 300 particles (now 0.47 ms).
-// Above, copying the arrays on the host first would cost more than that.
-constexpr size_t kStageBytes = 256 * 1024;
-
-struct hbtg_handle
+struct hbtg_handle : hbtg::Resources
 {
   int device = 0;
   int sm_count = 0;
-  cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;              // uploads that only the epilogue needs (host-pointer calls)
-  cudaStream_t side2 = nullptr;             // a second copy stream: velocities up, energies down
-  cudaEvent_t copy_events[7] = {};          // host-pointer calls: copy phases and the side streams
   cudaEvent_t epilogue_wait = nullptr;      // set for one call: the epilogue waits for this event
   Pool pool;
-  cudaEvent_t span[2] = {};                 // first and last event of a call
-  void *stage = nullptr;                    // pinned staging of small host-pointer calls, then of the totals
-  unsigned *ticket = nullptr;               // a device zero for the last-block scans (primitives.cuh)
   hbtg_stats stats{};
   bool count_interactions = false;
-  std::vector<cudaEvent_t> walk_events;
   std::vector<cudaEvent_t> phase_events; // phase boundaries of the last call, in order
   // learned warm start (hbtg_set_model)
   bool has_model = false;
@@ -1673,50 +1660,11 @@ int hbtg_create(hbtg_handle **handle, int device)
     return HBTG_ERR_NOMEM;
   h->device = device;
   h->sm_count = prop.multiProcessorCount;
-  if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) !=
-                                                  cudaSuccess)
+  const int rc = cudaSetDevice(device) == cudaSuccess ? h->create() : HBTG_ERR_CUDA;
+  if (rc != HBTG_OK)
   {
     delete h;
-    return HBTG_ERR_CUDA;
-  }
-  if (cudaMalloc(&h->ticket, 256) != cudaSuccess || cudaMemset(h->ticket, 0, 256) != cudaSuccess)
-  {
-    cudaGetLastError();
-    cudaFree(h->ticket);
-    cudaStreamDestroy(h->stream);
-    delete h;
-    return HBTG_ERR_NOMEM;
-  }
-  h->walk_events.resize(2);
-  for (auto &e : h->walk_events)
-    if (cudaEventCreate(&e) != cudaSuccess)
-    {
-      delete h;
-      return HBTG_ERR_CUDA;
-    }
-  if (cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&h->side2, cudaStreamNonBlocking) != cudaSuccess)
-  {
-    delete h;
-    return HBTG_ERR_CUDA;
-  }
-  for (auto &e : h->copy_events)
-    if (cudaEventCreate(&e) != cudaSuccess)
-    {
-      delete h;
-      return HBTG_ERR_CUDA;
-    }
-  for (auto &e : h->span)
-    if (cudaEventCreate(&e) != cudaSuccess)
-    {
-      delete h;
-      return HBTG_ERR_CUDA;
-    }
-  if (cudaMallocHost(&h->stage, kStageBytes + 256) != cudaSuccess)
-  {
-    cudaGetLastError();
-    delete h;
-    return HBTG_ERR_NOMEM;
+    return rc;
   }
   *handle = h;
   return HBTG_OK;
@@ -1728,23 +1676,9 @@ int hbtg_destroy(hbtg_handle *h)
     return HBTG_ERR_INVALID;
   cudaSetDevice(h->device);
   h->pool.release();
-  cudaFree(h->ticket);
-  cudaFreeHost(h->stage);
-  for (auto &e : h->span)
-    cudaEventDestroy(e);
-  for (auto &e : h->walk_events)
-    cudaEventDestroy(e);
   for (auto &e : h->phase_events)
     cudaEventDestroy(e);
-  for (auto &e : h->copy_events)
-    if (e)
-      cudaEventDestroy(e);
-  if (h->side)
-    cudaStreamDestroy(h->side);
-  if (h->side2)
-    cudaStreamDestroy(h->side2);
-  if (h->stream)
-    cudaStreamDestroy(h->stream);
+  h->release();
   delete h;
   return HBTG_OK;
 }
