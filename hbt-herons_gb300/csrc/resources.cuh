@@ -66,8 +66,10 @@ private:
     if (cudaMalloc(&p, 256) != cudaSuccess)
       return HBTG_ERR_NOMEM;
     ticket = static_cast<unsigned *>(p);
-    if (cudaMemset(ticket, 0, 256) != cudaSuccess)
-      return HBTG_ERR_NOMEM;
+    // zero before any stream can reach it: the streams here do not wait for the
+    // default stream, nor do the callers' own for these
+    if (cudaMemsetAsync(ticket, 0, 256, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
+      return HBTG_ERR_CUDA;
     for (cudaEvent_t &e : copy_events)
       if (cudaEventCreate(&e) != cudaSuccess)
         return HBTG_ERR_CUDA;

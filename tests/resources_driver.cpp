@@ -1,13 +1,14 @@
 // Drives csrc/resources.cuh against a runtime of its own that counts what is
 // live and can fail its n-th call.  Prints "live <objects left>" for a failed
-// creation, or for a whole one that was released again.
+// creation, or for a whole one that was released again, and "pending <streams>":
+// those with work enqueued that the creation did not wait for.
 #include <cstdio>
 #include <cstdlib>
 #include <set>
 
 #include "../hbt-herons_gb300/csrc/resources.cuh"
 
-static std::set<void *> live;
+static std::set<void *> live, pending;
 static int calls = 0, fail_at = -1;
 
 static bool fails() { return calls++ == fail_at; }
@@ -37,9 +38,17 @@ cudaError_t cudaMalloc(void **p, size_t) { return make(p); }
 cudaError_t cudaFree(void *p) { return drop(p); }
 cudaError_t cudaMallocHost(void **p, size_t) { return make(p); }
 cudaError_t cudaFreeHost(void *p) { return drop(p); }
-cudaError_t cudaMemset(void *, int, size_t) { return fails() ? cudaErrorInvalidValue : cudaSuccess; }
-cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t) { return fails() ? cudaErrorInvalidValue : cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return fails() ? cudaErrorUnknown : cudaSuccess; }
+cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t s)
+{
+  pending.insert(s);
+  return fails() ? cudaErrorInvalidValue : cudaSuccess;
+}
+cudaError_t cudaMemset(void *p, int v, size_t n) { return cudaMemsetAsync(p, v, n, nullptr); } // asynchronous on device memory
+cudaError_t cudaStreamSynchronize(cudaStream_t s)
+{
+  pending.erase(s);
+  return fails() ? cudaErrorUnknown : cudaSuccess;
+}
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 }
 
@@ -49,7 +58,8 @@ int main(int argc, char **argv)
   hbtg::Resources r;
   const int rc = r.create();
   const int made = calls;
+  const size_t waits = pending.size();
   if (rc == HBTG_OK)
     r.release();
-  std::printf("rc %d calls %d live %zu\n", rc, made, live.size());
+  std::printf("rc %d calls %d pending %zu live %zu\n", rc, made, waits, live.size());
 }

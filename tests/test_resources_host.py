@@ -31,3 +31,8 @@ def test_every_failure_is_cleaned_up(run):
     for k in range(calls):
         out = run(k)
         assert len(out) == 1 and not out[0].startswith("rc 0 ") and out[0].endswith("live 0"), (k, out)
+
+
+def test_nothing_is_pending_when_the_handle_is_returned(run):
+    """The ticket is zero before any stream, the caller's own included, can reach a kernel that takes it."""
+    assert " pending 0 " in run()[0]
