@@ -257,22 +257,26 @@ __global__ void k_re_leaves(ReState R, DevState D, int total)
   reinterpret_cast<int *>(&D.nodes[j + 2 * D.X[j] + 2 * D.cnt[j]])[3] = j;
 }
 
+// One axis offset a - b with the periodic wrap of the exact distance, rounded
+// once: the difference d and its own rounding error (two-sum) are exact, and so
+// is d -+ box for d within [box / 2, 2 box].  (Taking the box off a or b first is
+// exact only for coordinates inside the box.)
+__device__ __forceinline__ float re_offset(float a, float b, const ReState &R)
+{
+  const float d = __fsub_rn(a, b);
+  if (!R.periodic || !(fabsf(d) > R.half))
+    return d;
+  const float t = __fsub_rn(d, a), lost = __fsub_rn(__fsub_rn(a, __fsub_rn(d, t)), __fadd_rn(b, t));
+  return __fadd_rn(d > 0.f ? __fsub_rn(d, R.box) : __fadd_rn(d, R.box), lost);
+}
+
 // Squared distance in FP32 from the raw positions: within kReLoose (relative)
 // of the exact one.
 constexpr float kReLoose = 2e-6f;
 __device__ __forceinline__ float re_r2(const float4 &a, const float *q, const ReState &R)
 {
-  float d[3] = {__fsub_rn(a.x, q[0]), __fsub_rn(a.y, q[1]), __fsub_rn(a.z, q[2])};
-  if (R.periodic)
-  { // without rounding the large intermediate: one operand of a wrapped difference is beyond half the box
-    const float p[3] = {a.x, a.y, a.z};
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      d[k] = d[k] > R.half    ? __fsub_rn(__fsub_rn(p[k], R.box), q[k])
-             : d[k] < -R.half ? __fsub_rn(p[k], __fsub_rn(q[k], R.box))
-                              : d[k];
-  }
-  return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+  const float x = re_offset(a.x, q[0], R), y = re_offset(a.y, q[1], R), z = re_offset(a.z, q[2], R);
+  return x * x + y * y + z * z;
 }
 
 // Squared reach of a search whose k-th squared distance is at most r2: a cell
