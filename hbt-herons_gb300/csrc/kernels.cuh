@@ -680,29 +680,71 @@ __global__ void k_record_candidates(DevState D, int total)
   }
 }
 
-// Sum of floats with the rounding errors kept (two-sum): hi + lo is exact up
-// to the rounding of lo.
-struct PairSum
+// s += v; returns the addition's rounding error, exact (two-sum).
+__device__ __forceinline__ float two_sum(float &s, float v)
 {
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(float v)
-  {
-    const float t = __fadd_rn(hi, v), b = __fsub_rn(t, hi);
-    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
-    hi = t;
-  }
-  __device__ __forceinline__ void add(const PairSum &o)
+  const float t = __fadd_rn(s, v), b = __fsub_rn(t, s);
+  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(v, b));
+  s = t;
+  return e;
+}
+
+// Sum of floats in three words: the errors of `hi` are summed in `mid`, those of
+// that sum in `lo`, whose own rounding is some 2^-70 of the terms.  So value()
+// is at least as near as a sum in double (2^-53 an addition); two words, some
+// 2^-47, are not.
+struct FloatSum
+{
+  float hi = 0.f, mid = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(float v) { lo = __fadd_rn(lo, two_sum(mid, two_sum(hi, v))); }
+  __device__ __forceinline__ void add(const FloatSum &o)
   {
     add(o.hi);
-    lo = __fadd_rn(lo, o.lo);
+    lo = __fadd_rn(lo, __fadd_rn(two_sum(mid, o.mid), o.lo));
   }
-  // an infinite sum has no error term
-  __device__ __forceinline__ double value() const { return isfinite(lo) ? (double)hi + (double)lo : (double)hi; }
+  // an infinite sum has no error terms
+  __device__ __forceinline__ double value() const
+  {
+    return isfinite(mid) ? (double)hi + ((double)mid + (double)lo) : (double)hi;
+  }
 };
 
+// Sums of N quantities (a power of two) over the warp: lane l returns the total
+// of quantity l / (32 / N).  Each step halves what a lane still holds by handing
+// the other half to its partner, so 8 quantities take 9 additions, not 40.
+template <int N>
+__device__ __forceinline__ FloatSum warp_sums(FloatSum (&a)[N])
+{
+  const int lane = threadIdx.x & 31;
+  auto from = [](float hi, float mid, float lo, int o) {
+    FloatSum r;
+    r.hi = __shfl_xor_sync(0xffffffffu, hi, o);
+    r.mid = __shfl_xor_sync(0xffffffffu, mid, o);
+    r.lo = __shfl_xor_sync(0xffffffffu, lo, o);
+    return r;
+  };
+  int o = 16;
+#pragma unroll
+  for (int h = N / 2; h > 0; h >>= 1, o >>= 1)
+#pragma unroll
+    for (int i = 0; i < h; i++)
+    {
+      const bool up = (lane & o) != 0;
+      FloatSum &x = a[i], &y = a[i + h]; // (word by word: a choice between the structs would put them in memory)
+      const FloatSum give = from(up ? x.hi : y.hi, up ? x.mid : y.mid, up ? x.lo : y.lo, o);
+      x.hi = up ? y.hi : x.hi;
+      x.mid = up ? y.mid : x.mid;
+      x.lo = up ? y.lo : x.lo;
+      x.add(give);
+    }
+#pragma unroll
+  for (; o > 0; o >>= 1)
+    a[0].add(from(a[0].hi, a[0].mid, a[0].lo, o));
+  return a[0];
+}
+
 // The sums, over the particles packed by part_off: a warp takes 256
-// consecutive ones and keeps its lanes' sums per type in error-free float
-// pairs until the subhalo or the part changes.  One block per subhalo, with
+// consecutive ones and keeps its lanes' sums per type in FloatSums until the subhalo or the part changes.  One block per subhalo, with
 // FP64 sums, took 0.81 ms for a subhalo of 1.4e5 particles (2.4 of the 13.2 ms
 // of a 1e6-particle subsampled call, which this brought to 12.2 ms).
 constexpr int kUpscaleRows = 8;
@@ -712,24 +754,18 @@ __global__ void __launch_bounds__(256) k_upscale_sums(DevState D, KParams K, int
   const long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kUpscaleRows * kWarp);
   if (first >= total) // whole warps
     return;
-  PairSum acc[6];
+  FloatSum acc[6];
   int cur_s = -1, cur_part = 0; // what acc belongs to
   auto hand_in = [&](int s, int part, bool in) {
+    FloatSum v[8];
 #pragma unroll
     for (int t = 0; t < 6; t++)
-    {
-      if (!__any_sync(0xffffffffu, in && acc[t].hi != 0.f))
-        continue;
-      PairSum v;
       if (in)
-        v = acc[t];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-        v.add(PairSum{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
-      if (lane == 0)
-        atomicAdd(part == 2 ? upscale_sub(D, s) + 6 : part == 0 ? upscale_sub(D, s) + t : upscale_rest(D, s) + t,
-                  v.value());
-    }
+        v[t] = acc[t];
+    const double sum = warp_sums(v).value();
+    const int t = lane >> 2;
+    if ((lane & 3) == 0 && t < 6 && sum != 0.)
+      atomicAdd(part == 2 ? upscale_sub(D, s) + 6 : part == 0 ? upscale_sub(D, s) + t : upscale_rest(D, s) + t, sum);
   };
 #pragma unroll 1
   for (int r = 0; r < kUpscaleRows; r++)
@@ -756,7 +792,7 @@ __global__ void __launch_bounds__(256) k_upscale_sums(DevState D, KParams K, int
         hand_in(cur_s, cur_part, true);
 #pragma unroll
       for (int t = 0; t < 6; t++)
-        acc[t] = PairSum();
+        acc[t] = FloatSum();
       cur_s = one ? s0 : -1;
       cur_part = p0;
     }
@@ -776,7 +812,7 @@ __global__ void __launch_bounds__(256) k_upscale_sums(DevState D, KParams K, int
       }
 #pragma unroll
       for (int t = 0; t < 6; t++)
-        acc[t] = PairSum();
+        acc[t] = FloatSum();
     }
   }
   if (cur_s >= 0)

@@ -6,8 +6,8 @@
 //
 // The bound particles of every subhalo are packed (item j = bound position k
 // of subhalo s).  One pass computes each item's distance from the most-bound
-// particle and its shape terms (summed per subhalo in float pairs, TwoSum, and
-// those in double); the items are
+// particle and its shape terms (summed per subhalo in FloatSums, and those
+// in double); the items are
 // then sorted by distance within their subhalo (radix sort by distance, then
 // stably by subhalo), the cumulative masses come from one segmented scan in
 // double, and the profile quantities from per-subhalo reductions over the
@@ -82,30 +82,23 @@ __global__ void k_prop_init(PropState P)
     P.shape[12 * s + q] = 0.;
 }
 
-// Adds a warp's 12 pair sums over the lanes with `in` to subhalo seg's shape.
-__device__ __forceinline__ void add_shape(const PropState &P, int seg, bool in, PairSum (&acc)[12])
+// Adds a warp's 12 sums over the lanes with `in` to subhalo seg's shape.
+__device__ __forceinline__ void add_shape(const PropState &P, int seg, bool in, const FloatSum (&acc)[12])
 {
-  const int lane = threadIdx.x & 31;
-  double mine = 0.;
+  const int lane = threadIdx.x & 31, q = lane >> 1;
+  FloatSum t[16];
 #pragma unroll
-  for (int q = 0; q < 12; q++)
-  {
-    PairSum t;
+  for (int k = 0; k < 12; k++)
     if (in)
-      t = acc[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      t.add(PairSum{__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o)});
-    if (lane == q)
-      mine = t.value();
-  }
-  if (lane < 12 && mine != 0.)
-    atomicAdd(&P.shape[12 * seg + lane], mine);
+      t[k] = acc[k];
+  const double sum = warp_sums(t).value();
+  if ((lane & 1) == 0 && q < 12 && sum != 0.)
+    atomicAdd(&P.shape[12 * seg + q], sum);
 }
 
 // Items: distances, masses, sort keys; shape sums (CalculateShape skips the
 // first bound particle, the centre itself).  A warp takes kPropRows rows of 32
-// consecutive items and keeps the 12 sums in error-free float pairs (FP64 is
+// consecutive items and keeps the 12 sums in FloatSums (FP64 is
 // scarce on this GPU: 24 operations an item held this kernel at 443 us on
 // 3.3e6 items, with 16 strided items a thread) until the subhalo changes;
 // then one double atomic per sum.  Bound by the gathers of positions and
@@ -117,7 +110,7 @@ __global__ void __launch_bounds__(256) k_prop_items(PropState P, int total)
   const long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kPropRows * kWarp);
   if (first >= total) // whole warps
     return;
-  PairSum acc[12];
+  FloatSum acc[12];
   int cur = -1; // subhalo that acc belongs to
 #pragma unroll 1
   for (int r = 0; r < kPropRows; r++)
@@ -161,7 +154,7 @@ __global__ void __launch_bounds__(256) k_prop_items(PropState P, int total)
         add_shape(P, cur, true, acc);
 #pragma unroll
       for (int q = 0; q < 12; q++)
-        acc[q] = PairSum();
+        acc[q] = FloatSum();
       cur = one ? s0 : -1;
     }
     if (counts)
@@ -178,7 +171,7 @@ __global__ void __launch_bounds__(256) k_prop_items(PropState P, int total)
       }
 #pragma unroll
       for (int q = 0; q < 12; q++)
-        acc[q] = PairSum();
+        acc[q] = FloatSum();
     }
   }
   if (cur >= 0)

@@ -12,12 +12,14 @@
 //
 // Every step is the lock-step one (kernels.cuh has the reference's lines):
 // the same keys in the same stable order, the same tree, the same chunks of
-// 32 targets walked by the same code, the same energies and partition; so the
-// results are the same bits.  The centre-of-mass sums are the one place where
-// grouping could show: k_com adds single items in double once an iteration's
-// bound sets hold at most kComSmall particles, which any order reproduces to
-// ~1e-16 of the sum, so teams (which add error-free float pairs) take over
-// only from there on (IterationDriver::iterate).
+// 32 targets walked by the same code, the same energies and partition.  The
+// centre-of-mass sums are the one place where grouping could show: k_com adds
+// single items in double once an iteration's bound sets hold at most kComSmall
+// particles, some 1e-16 of the summed magnitudes off whatever its order, and
+// teams (which add three-word FloatSums, then a double per warp) take over only
+// from there on (IterationDriver::iterate).  So both round to the same float
+// unless the sum lies within that of a halfway point: the results are the same
+// bits in every case tried, and expected to be, but not by construction.
 //
 // Limits of a team: kSettleSrc tree sources (their keys and tree indices lie
 // in shared memory), kSettleSlots tree slots, and no potential subsample.  A
@@ -669,7 +671,7 @@ __global__ void __launch_bounds__(settle_threads(C), C == 1 ? 3 : 1) k_settle(De
       // centre-of-mass frame (k_com, frame_from_sums)
       {
         const float4 o = D.pm[ord[0]];
-        PairSum acc[7];
+        FloatSum acc[8]; // the last one is padding
         for (int k = gtid; k < nb; k += kTeam)
         {
           const int p = ord[k];
@@ -684,16 +686,9 @@ __global__ void __launch_bounds__(settle_threads(C), C == 1 ? 3 : 1) k_settle(De
           acc[5].add(__fmul_rn(v.y, mass));
           acc[6].add(__fmul_rn(v.z, mass));
         }
-#pragma unroll
-        for (int c = 0; c < 7; c++)
-        {
-          PairSum v = acc[c];
-#pragma unroll
-          for (int h = 16; h > 0; h >>= 1)
-            v.add(PairSum{__shfl_xor_sync(0xffffffffu, v.hi, h), __shfl_xor_sync(0xffffffffu, v.lo, h)});
-          if (lane == 0)
-            dsum[w][c] = v.value();
-        }
+        const double sum = warp_sums(acc).value();
+        if ((lane & 3) == 0 && lane < 28)
+          dsum[w][lane >> 2] = sum;
         __syncthreads();
         if (tid < 7)
         {
