@@ -408,7 +408,7 @@ struct IterationDriver
       { // upscale factors of the subsampled subhaloes
         if (part_total > 0)
           k_upscale_sums<<<grid_for((part_total + kUpscaleRows - 1) / kUpscaleRows, 256), 256, 0, st>>>(D, K, part_total);
-        k_upscale<<<sb, 256, 0, st>>>(D, K);
+        k_upscale<<<grid_for((long long)S * kWarp, 256), 256, 0, st>>>(D, K);
         launches += 2;
         check();
       }

@@ -743,29 +743,58 @@ __device__ __forceinline__ FloatSum warp_sums(FloatSum (&a)[N])
   return a[0];
 }
 
-// The sums, over the particles packed by part_off: a warp takes 256
-// consecutive ones and keeps its lanes' sums per type in FloatSums until the subhalo or the part changes.  One block per subhalo, with
-// FP64 sums, took 0.81 ms for a subhalo of 1.4e5 particles (2.4 of the 13.2 ms
-// of a 1e6-particle subsampled call, which this brought to 12.2 ms).
-constexpr int kUpscaleRows = 8;
+// Part `pos` (0 exempt, 1 sources, 2 the others) of sampled subhalo s: its range
+// [a, b) of packed items.
+__device__ __forceinline__ void upscale_part(const DevState &D, const KParams &K, int s, int pos, int &a, int &b)
+{
+  const int first = D.part_off[s], exempt = first + D.nunsample[s], sample = exempt + K.max_sample;
+  a = pos == 0 ? first : pos == 1 ? exempt : sample;
+  b = pos == 0 ? exempt : pos == 1 ? sample : D.part_off[s + 1];
+}
+// Sums [2 w], [2 w + 1] of warp w over the first and the last part it shares with
+// its neighbours, six types each; the keys are free until the tree build.
+__device__ __forceinline__ double *upscale_partial(const DevState &D, int i)
+{
+  return reinterpret_cast<double *>(D.key) + 6 * (size_t)i;
+}
+
+// The sums, over the particles packed by part_off: a warp takes kUpscaleItems
+// consecutive ones and keeps its lanes' sums per type in FloatSums until the
+// subhalo or the part changes.  A part that lies within one warp's items is
+// stored, the pieces of a longer one go to k_upscale, which adds them in order,
+// so a call gives the same factors every time.  One block per subhalo, with FP64
+// sums, took 0.81 ms for a subhalo of 1.4e5 particles (2.4 of the 13.2 ms of a
+// 1e6-particle subsampled call, which this brought to 12.2 ms).
+constexpr int kUpscaleRows = 8, kUpscaleItems = kUpscaleRows * kWarp;
 __global__ void __launch_bounds__(256) k_upscale_sums(DevState D, KParams K, int total)
 {
   const int lane = threadIdx.x & 31;
-  const long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kUpscaleRows * kWarp);
+  const int w = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const long long first = (long long)w * kUpscaleItems;
   if (first >= total) // whole warps
     return;
   FloatSum acc[6];
-  int cur_s = -1, cur_part = 0; // what acc belongs to
-  auto hand_in = [&](int s, int part, bool in) {
+  int cur = -1; // the part that acc belongs to: 3 s + pos
+  auto hand_in = [&]() {
+    const int s = cur / 3, pos = cur - 3 * s;
+    if (D.corr[s] || D.ngrav[s] == 0)
+      return;
     FloatSum v[8];
 #pragma unroll
     for (int t = 0; t < 6; t++)
-      if (in)
-        v[t] = acc[t];
+      v[t] = acc[t];
     const double sum = warp_sums(v).value();
     const int t = lane >> 2;
-    if ((lane & 3) == 0 && t < 6 && sum != 0.)
-      atomicAdd(part == 2 ? upscale_sub(D, s) + 6 : part == 0 ? upscale_sub(D, s) + t : upscale_rest(D, s) + t, sum);
+    if ((lane & 3) != 0 || t >= 6)
+      return;
+    int a, b;
+    upscale_part(D, K, s, pos, a, b);
+    if (a < first || b > first + kUpscaleItems)
+      upscale_partial(D, 2 * w + (a < first ? 0 : 1))[t] = sum;
+    else if (pos != 0)
+      (pos == 1 ? upscale_sub(D, s) : upscale_rest(D, s))[t] = sum;
+    else if (t == 0)
+      upscale_sub(D, s)[6] = sum;
   };
 #pragma unroll 1
   for (int r = 0; r < kUpscaleRows; r++)
@@ -775,59 +804,79 @@ __global__ void __launch_bounds__(256) k_upscale_sums(DevState D, KParams K, int
     const int s = find_segment_warp(D.part_off, D.S, j);
     const bool in = jj < total && !D.corr[s] && D.ngrav[s] != 0;
     const int k = j - D.part_off[s], ns = D.nunsample[s];
-    const int part = k < ns ? 2 : (k < ns + K.max_sample ? 0 : 1);
+    const int pos = k < ns ? 0 : (k < ns + K.max_sample ? 1 : 2);
     float m = 0.f;
     int ty = 7;
     if (in)
     {
       const int p = D.ord[D.off[s] + k];
       m = D.pm[p].w;
-      ty = D.ty[p] & 7;
+      ty = pos == 0 ? 0 : D.ty[p] & 7; // of the exempt ones the types do not matter
     }
-    const int s0 = __shfl_sync(0xffffffffu, s, 0), p0 = __shfl_sync(0xffffffffu, part, 0);
-    const bool one = __all_sync(0xffffffffu, s == s0 && part == p0);
-    if (!one || s0 != cur_s || p0 != cur_part)
+    const int part = 3 * s + pos; // never decreasing over the lanes and rows
+    for (unsigned left = 0xffffffffu; left;)
     {
-      if (cur_s >= 0)
-        hand_in(cur_s, cur_part, true);
-#pragma unroll
-      for (int t = 0; t < 6; t++)
-        acc[t] = FloatSum();
-      cur_s = one ? s0 : -1;
-      cur_part = p0;
-    }
-#pragma unroll
-    for (int t = 0; t < 6; t++)
-      if (ty == t)
-        acc[t].add(m);
-    if (!one)
-    { // each subhalo and part of the row by itself
-      for (unsigned left = 0xffffffffu; left;)
+      const int now = __shfl_sync(0xffffffffu, part, __ffs(left) - 1);
+      const bool mine = part == now;
+      left &= ~__ballot_sync(0xffffffffu, mine);
+      if (now != cur)
       {
-        const int src = __ffs(left) - 1;
-        const int sl = __shfl_sync(0xffffffffu, s, src), pl = __shfl_sync(0xffffffffu, part, src);
-        const bool mine = s == sl && part == pl;
-        left &= ~__ballot_sync(0xffffffffu, mine);
-        hand_in(sl, pl, mine);
+        if (cur >= 0)
+          hand_in();
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+          acc[t] = FloatSum();
+        cur = now;
       }
 #pragma unroll
       for (int t = 0; t < 6; t++)
-        acc[t] = FloatSum();
+        if (mine && ty == t)
+          acc[t].add(m);
     }
   }
-  if (cur_s >= 0)
-    hand_in(cur_s, cur_part, true);
+  hand_in();
 }
 
 // Mass upscale factors of the subsampled subhaloes from their sums
 // (GetMassUpscaleFactor[PerParticleType], src/subhalo_unbind.cpp:290-361), by
-// the reference's float formulas.
+// the reference's float formulas.  A warp per subhalo, for the pieces of its sums.
 __global__ void k_upscale(DevState D, KParams K)
 {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= D.S || D.state[s] != kActive || D.corr[s] || !D.ngrav[s])
+  const int s = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (s >= D.S || D.state[s] != kActive || D.corr[s] || !D.ngrav[s]) // whole warps
     return;
-  const double *sub_m = upscale_sub(D, s), *rest = upscale_rest(D, s);
+  double *sub_m = upscale_sub(D, s), *rest = upscale_rest(D, s);
+  for (int pos = 0; pos < 3; pos++)
+  {
+    int a, b;
+    upscale_part(D, K, s, pos, a, b);
+    const int w0 = a / kUpscaleItems, w1 = (b - 1) / kUpscaleItems;
+    if (b <= a || w0 == w1)
+      continue;
+    double v[6] = {0., 0., 0., 0., 0., 0.};
+    for (int w = w0 + lane; w <= w1; w += kWarp)
+    {
+      const double *p = upscale_partial(D, 2 * w + (w == w0 ? 1 : 0));
+#pragma unroll
+      for (int t = 0; t < 6; t++)
+        v[t] += p[t];
+    }
+#pragma unroll
+    for (int t = 0; t < 6; t++)
+      for (int o = 16; o > 0; o >>= 1)
+        v[t] += __shfl_xor_sync(0xffffffffu, v[t], o);
+    if (lane == 0)
+    {
+      if (pos == 0)
+        sub_m[6] = v[0];
+      else
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+          (pos == 1 ? sub_m : rest)[t] = v[t];
+    }
+  }
+  if (lane != 0)
+    return;
   float f[6];
   if (!K.dm_only && K.upscale_per_type)
   {
