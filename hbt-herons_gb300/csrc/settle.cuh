@@ -53,15 +53,18 @@ constexpr int kSettleSlots = 8192;  // tree slots of a block (each block of a cl
 constexpr int kSettleCluster = 8;   // blocks of a cluster's team
 // Targets up to which one block takes a subhalo (a chunk of 32 per warp, or
 // four in the correction loop or when there are more of that size than
-// clusters), and a cluster; above, the grid: its barriers cost most (some 3 us), and it takes one subhalo at a
-// time.  One of 46,000 particles with 50 iterations left took 34 ms with a
-// cluster's 64 warps, 31 ms in lock step and 15 ms with the grid.
-constexpr int kSettleSmall = 256, kSettleOne = 1024, kSettleMid = 8192;
+// clusters), and a cluster; above kSettleMid, the grid, whose barriers cost most (some 3 us) and which takes one
+// subhalo at a time.  One of 46,000 particles with 50 iterations left took 34 ms with a
+// cluster's 64 warps, 31 ms in lock step and 15 ms with the grid.  Several of up to kSettleLarge go to clusters all
+// the same, which take them side by side: six of 16,000 particles take a call of 10.4 ms one after the other, 3.5 ms
+// with clusters and 3.8 ms in lock step; one alone 2.95, 2.99 and 3.03 ms.  Two of 30,000: 2.4 to 3.5 ms with the
+// grid, 3.1 to 4.4 ms with clusters; three of 20,000: 3.1 to 4.0 and 3.3 to 4.1 (more do not fit into the 65,536).
+constexpr int kSettleSmall = 256, kSettleOne = 1024, kSettleMid = 8192, kSettleLarge = 20480;
 constexpr int kSettleTeams1 = 456, kSettleTeams8 = 38; // most teams of one launch (3 blocks fit an SM)
 constexpr int kSettleMaxBlocks = 1024;                  // of a team (the grid's)
 enum SettleClass : int
 {
-  kSettleA, kSettleB, kSettleC, kSettleD, // by the three limits above
+  kSettleA, kSettleB, kSettleC, kSettleD, kSettleE, // by the four limits above
   kSettleClasses
 };
 
@@ -115,7 +118,7 @@ __global__ void k_settle_pick(DevState D, KParams K, SettleArgs A)
   if (sampled || (D.corr[s] ? D.nlast[s] - n : n) > kSettleSrc)
     return;
   // (the correction loop's trees are small: a block's barriers are cheaper there than a cluster's warps)
-  const int c = n <= kSettleSmall || (n <= kSettleOne && D.corr[s]) ? kSettleA : n <= kSettleOne ? kSettleB : n <= kSettleMid ? kSettleC : kSettleD;
+  const int c = n <= kSettleSmall || (n <= kSettleOne && D.corr[s]) ? kSettleA : n <= kSettleOne ? kSettleB : n <= kSettleMid ? kSettleC : n <= kSettleLarge ? kSettleD : kSettleE;
   A.list[(size_t)c * D.S + atomicAdd(&A.count[c], 1)] = s;
 }
 
@@ -449,16 +452,20 @@ __global__ void __launch_bounds__(settle_threads(C), C == 1 ? 3 : 1) k_settle(De
   const int blocks = C == kGrid ? (int)gridDim.x : C; // of the team
   const int rank = (int)blockIdx.x % blocks, team = (int)blockIdx.x / blocks, teams = (int)gridDim.x / blocks;
   const int gtid = rank * kSettleThreads + tid, kTeam = blocks * kSettleThreads;
-  // this kernel's subhaloes: one or two of the classes
-  const bool b_large = A.count[kSettleB] <= kSettleTeams8; // class B to the clusters
-  const int c0 = C == 1 ? kSettleA : C == kGrid ? kSettleD : kSettleC;
-  const int n0 = A.count[c0], n1 = C != kGrid && b_large == (C > 1) ? A.count[kSettleB] : 0, count = n0 + n1;
+  // this kernel's subhaloes: up to three of the classes, one after the other
+  const bool b_large = A.count[kSettleB] <= kSettleTeams8;               // class B to the clusters
+  const bool d_alone = A.count[kSettleD] + A.count[kSettleE] == 1;       // class D to the grid
+  const int c0 = C == 1 ? kSettleA : C == kGrid ? kSettleE : kSettleC;
+  const int n0 = A.count[c0], n1 = C != kGrid && b_large == (C > 1) ? A.count[kSettleB] : 0,
+            n2 = C != 1 && d_alone == (C == kGrid) ? A.count[kSettleD] : 0, count = n0 + n1 + n2;
   float4 *const slots = A.nodes + (size_t)blockIdx.x * kSettleSlots;
   double *xch = A.xch + (size_t)team * 2 * blocks * 8;
   int par = 0, xpar = 0; // alternating halves of `part` / wcnt and of xch
   for (int q = team; q < count; q += teams)
   {
-    const int s = q < n0 ? A.list[(size_t)c0 * D.S + q] : A.list[(size_t)kSettleB * D.S + (q - n0)];
+    const int s = q < n0        ? A.list[(size_t)c0 * D.S + q]
+                  : q < n0 + n1 ? A.list[(size_t)kSettleB * D.S + (q - n0)]
+                                : A.list[(size_t)kSettleD * D.S + (q - n0 - n1)];
     const long long off = D.off[s];
     int *ord = D.ord + off, *ord_tmp = D.ord_tmp + off;
     int nbound = D.nbound[s], nlast = D.nlast[s], corr = D.corr[s], iter = D.iter[s], wrap = D.wrap[s];
