@@ -29,6 +29,7 @@
 #include "kernels.cuh"
 #include "primitives.cuh"
 #include "settle.cuh"
+#include "stream_sms.cuh"
 #include "walk.cuh"
 
 namespace hbtg
@@ -61,6 +62,7 @@ struct IterationDriver
   int64_t host_syncs = 0; // stream synchronisations for host reads of device totals
   int global_iter = 0;
   bool teams = true;    // false once there was no room for their buffers
+  int grid_team = -1;   // blocks of the grid's team (-1: not asked yet, 0: the stream has no room for one)
   int settle_from = -1; // lock-step iterations before the first k_settle of the call (-1: none)
   SettleArgs settle_args{};
 
@@ -319,7 +321,8 @@ struct IterationDriver
   void settle(long long live)
   {
     SettleArgs &A = settle_args;
-    if (!mem.settle_buffers(A, S, live > kSettleMid ? settle_grid() : 0))
+    A.grid = live > kSettleMid ? settle_grid() : 0; // else no subhalo is that large
+    if (!mem.settle_buffers(A, S, A.grid))
     {
       teams = false;
       return;
@@ -334,9 +337,10 @@ struct IterationDriver
     k_settle_pick<<<grid_for(S, 256), 256, 0, st>>>(D, K, A);
     launch_settle<1>(std::min(S, kSettleTeams1));
     launch_settle<kSettleCluster>(std::min(S, kSettleTeams8) * kSettleCluster);
-    if (live > kSettleMid) // else no subhalo is that large
+    if (A.grid > 0)
     {
-      launch_settle<kGrid>(settle_grid());
+      if (!launch_settle<kGrid>(A.grid))
+        grid_team = 0;
       launches++;
     }
     launches += 3;
@@ -344,11 +348,25 @@ struct IterationDriver
     mem.mark(1);
   }
 
-  // Blocks of the grid's team, one per SM: all are resident.
-  int settle_grid() const { return std::min(kSettleMaxBlocks, sm_count); }
+  // Blocks of the grid's team, one per SM that the stream can use: all have to
+  // be resident at once, or the launch is refused.  Zero: its subhaloes go to
+  // clusters or stay in lock step.
+  int settle_grid()
+  {
+    if (grid_team < 0)
+    {
+      const int smem = (int)sizeof(SettleShared<kGrid>);
+      int per_sm = 0;
+      mem.check(cudaFuncSetAttribute(k_settle<kGrid>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      mem.check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_settle<kGrid>, settle_threads(kGrid), smem));
+      grid_team = per_sm > 0 ? std::min(kSettleMaxBlocks, stream_sms(st, sm_count)) : 0;
+    }
+    return grid_team;
+  }
 
+  // False: the grid's team was refused for want of room.
   template <int C>
-  void launch_settle(int blocks)
+  bool launch_settle(int blocks)
   {
     const int smem = (int)sizeof(SettleShared<C>);
     mem.check(cudaFuncSetAttribute(k_settle<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -371,7 +389,14 @@ struct IterationDriver
     }
     cfg.attrs = attr;
     cfg.numAttrs = C != 1 ? 1 : 0;
-    mem.check(cudaLaunchKernelEx(&cfg, k_settle<C>, D, K, settle_args));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_settle<C>, D, K, settle_args);
+    if (C == kGrid && e == cudaErrorCooperativeLaunchTooLarge)
+    {
+      cudaGetLastError();
+      return false;
+    }
+    mem.check(e);
+    return true;
   }
 
   void run()

@@ -78,6 +78,7 @@ struct SettleArgs
   double *xch;              // [2][blocks of the team][8] per team: sums in exchange between its blocks
   unsigned long long *cells; // tree cells built
   int *most;                 // most iterations that one subhalo took here
+  int grid;                  // blocks of the grid's team (0: none)
 };
 
 // Arrays of a block that live between two walks (the walk's lists take their place).
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(settle_threads(C), C == 1 ? 3 : 1) k_settle(De
   const int gtid = rank * kSettleThreads + tid, kTeam = blocks * kSettleThreads;
   // this kernel's subhaloes: up to three of the classes, one after the other
   const bool b_large = A.count[kSettleB] <= kSettleTeams8;               // class B to the clusters
-  const bool d_alone = A.count[kSettleD] + A.count[kSettleE] == 1;       // class D to the grid
+  const bool d_alone = A.grid && A.count[kSettleD] + A.count[kSettleE] == 1; // class D to the grid
   const int c0 = C == 1 ? kSettleA : C == kGrid ? kSettleE : kSettleC;
   const int n0 = A.count[c0], n1 = C != kGrid && b_large == (C > 1) ? A.count[kSettleB] : 0,
             n2 = C != 1 && d_alone == (C == kGrid) ? A.count[kSettleD] : 0, count = n0 + n1 + n2;
