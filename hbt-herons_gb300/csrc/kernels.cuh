@@ -2093,7 +2093,8 @@ __global__ void k_epi_core(DevState D, KParams K, float *core)
     return;
   }
   const int *ord = D.ord + D.off[s];
-  const long long core_size = max((long long)((float)nb * K.core_factor), K.core_min);
+  const long long asked = max((long long)((float)nb * K.core_factor), K.core_min);
+  const long long core_size = asked < 0 ? 2ll * nb : asked; // a size never reached takes every particle
   const float4 x0 = D.pm[ord[0]];
   const double org[3] = {K.periodic ? (double)x0.x : 0., K.periodic ? (double)x0.y : 0., K.periodic ? (double)x0.z : 0.};
   double q[13]; // mass, then first and second moments of position and velocity
