@@ -69,8 +69,8 @@
 // over half of it in the traversal.  So a step has one path for every lane
 // (lanes without a range read the last one again), the three lists share one
 // layout and one write, a warp's arrays lie together behind one base address,
-// and the far terms use the reciprocal square root without the steps for
-// subnormal arguments.  Against a version with separate lists, per-kind
+// and the far terms use the PTX reciprocal square root that takes normal
+// arguments only (rsqrt_normal).  Against a version with separate lists, per-kind
 // branches and rsqrtf, on the 5e7-particle learned batch: 137.4 -> 123.7 ms a
 // call; on a 5e6-particle plain batch with a halo across a box face 31.1 ->
 // 29.0 ms (walk 20.9 -> 16.6 ms); a subsampled hydro call 23.5 -> 21.0 ms.
@@ -307,9 +307,10 @@ __device__ __forceinline__ void box_dist2(const float *lo, const float *hi, floa
   far2 = dist2(fmaxf(fabsf(l[0]), fabsf(h[0])), fmaxf(fabsf(l[1]), fabsf(h[1])), fmaxf(fabsf(l[2]), fabsf(h[2])));
 }
 
-// 1 / sqrt of a number that is not subnormal: the approximation that rsqrtf
-// returns there, without the steps that scale a subnormal argument (three of
-// its four instructions).
+// 1 / sqrt of a positive number that is not subnormal.  The PTX instruction is
+// documented to be within 2^-22.9 (relative) over the positive floats, and with
+// .ftz to take a subnormal argument for zero; the far entries lie beyond the
+// softening length, so their squared distances are at least h2s, which is normal.
 __device__ __forceinline__ float rsqrt_normal(float x)
 {
   float r;
