@@ -1157,7 +1157,10 @@ __device__ __forceinline__ void cell_bounds(float4 *nodes, int slot)
 // grid.  Cluster = true: a run of levels of few cells on one cluster, a
 // barrier (which orders the blocks' global accesses) between levels.  A small
 // level is bound by the latency of its start and of its chain of children:
-// 11 us as a launch of its own, 6 us in a run.
+// 11 us as a launch of its own, 6 us in a run.  A run's levels hold at most
+// kMomentsFew cells: with no runs, this limit and one of 65,536 a halo of 1e5
+// takes 2.55, 2.50 and 2.55 ms, of 1e6 6.70, 6.67 and 6.82, a plain batch of
+// 1e6 particles 8.88, 8.78 and 9.17.
 struct LevelOffsets
 {
   int off[kLevels];
@@ -2076,7 +2079,9 @@ __device__ __forceinline__ void put_core(float *cr, double msum, const double *p
 // calls on at most kCoreWarps subhaloes: one thread's chain of loads and FP64
 // operations over the twenty particles of a core was 40 of k_epilogue's 55 us,
 // and most of a call's latency has nothing beside it.  With more subhaloes a
-// thread each does the same work with fewer FP64 instructions.
+// thread each does the same work with fewer FP64 instructions: the final phase
+// of 4,000 subhaloes of 25 to 40 particles takes 0.264 ms by warps and 0.284 by
+// threads, of 8,000 0.318 and 0.292, of 16,000 0.390 and 0.319.
 constexpr int kCoreWarps = 4096;
 __global__ void k_epi_core(DevState D, KParams K, float *core)
 {

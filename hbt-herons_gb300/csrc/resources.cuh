@@ -14,8 +14,10 @@ namespace hbtg
 
 // Host-pointer calls whose arrays take at most this much go through one pinned
 // buffer and one copy each way: some thirty copies of a few hundred bytes were
-// 0.2 ms of a 0.65 ms call on one subhalo of 300 particles (now 0.47 ms).
-// Above, copying the arrays on the host first would cost more than that.
+// 0.2 ms of a 0.65 ms call on one subhalo of 300 particles (now 0.47 ms), and of
+// 4,000, the largest that fit, 1.26 ms (now 1.12).  The limit is the pinned
+// memory that a handle holds: a buffer of 8 MB would still take a call on 6,000
+// particles from 1.36 to 1.19 ms, on 16,000 from 1.69 to 1.52, on 32,000 from 2.03 to 1.93.
 constexpr size_t kStageBytes = 256 * 1024;
 
 struct Resources
