@@ -484,6 +484,8 @@ def bench_gpu(args):
                                              "plain": plain and plain["counted"]["global_iterations"]},
                        "interactions_per_step": {"learned": cw["interactions"],
                                                  "plain": plain and plain["counted"]["interactions"]},
+                       # a call that counts stays in lock step to its end: the counts below are its, not a timed step's
+                       "counted_call": "lock step to the end (timed steps hand their late iterations to teams)",
                        "walk_traversal_per_step": {k[5:]: cw[k] for k in (
                            "walk_steps", "walk_nodes", "walk_pending_batches", "walk_entries_full",
                            "walk_entries_part", "walk_entries_near", "walk_drained")},
@@ -516,7 +518,10 @@ def bench_gpu(args):
                          "blocks_per_sm": warm["last"].get("walk_blocks_per_sm"),
                          "issue_active_ncu": issue,
                          "bound_note": "the walk is issue-bound (instruction issue slots, not the FP32 pipe): "
-                                       "issue_active_ncu is its ncu issue-slot utilisation",
+                                       "issue_active_ncu is its ncu issue-slot utilisation; ms_per_launch is the "
+                                       "walks' and the late iterations' teams' whole time (trees, sorts and frames "
+                                       "among it) over a timed step's walk launches, the interactions are those of "
+                                       "a lock-step call",
                          "walk_share_of_step": warm["ms_walk"] / max(warm["ms"], 1e-9)},
             "cpu_baseline": cpu,
             "parity": parity,
