@@ -40,9 +40,9 @@ def test_six_large_subhaloes(unbinder):
     assert ms[6] < 2 * ms[1], ms
 
 
-@pytest.mark.parametrize("sizes", [(8192, 8193), (9000,) * 6, (20_480,), (20_481, 9000), (21_000, 20_480, 8193)])
+@pytest.mark.parametrize("sizes", [(256,), (257,), (1024,), (1025,), (1024,) * 50, (8192, 8193), (9000,) * 6, (20_480,), (20_481, 9000), (21_000, 20_480, 8193)])
 def test_the_same_bits_whichever_team(unbinder, sizes):
-    """Sizes about the limits between clusters and the grid, alone and several, against lock step."""
+    """Sizes about the limits between blocks, clusters and the grid, alone and several, against lock step."""
     prm = abi.parity_params(dm_only=1, box_size=500.0)
     parts = [synthetic.stripped(n_sub=1, seed=3 + k, nmin=n, nmax=n + 1) for k, n in enumerate(sizes)]
     cat = lambda k: np.concatenate([getattr(p, k) for p in parts])  # noqa: E731
